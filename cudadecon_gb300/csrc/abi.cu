@@ -291,12 +291,15 @@ static int fill_otf(GridPlan& p, float dr, float dz, const OtfSpec& o, cudaStrea
   od.kxscale = dkx / o.dkx_otf;
   od.kyscale = dky / o.dky_otf;
   od.kzscale = dkz / o.dkz_otf;
-  const float scale = (float)(1.0 / ((double)gx * gy * gz));
+  // the paired passes' spectrum is twice the transform
+  choose_layout(p.g, p.fx, p.fy);
+  const float scale = (float)((p.g.pair ? 0.5 : 1.0) / ((double)gx * gy * gz));
   p.otf.nr = od.nx_otf;
   p.otf.kxscale = od.kxscale;
   p.otf.kyscale = od.kyscale;
   p.otf.tz = nullptr;
   p.otf.full = nullptr;
+  p.otf.h0 = reinterpret_cast<const float*>(o.raw_otf);
   int rc;
   if (od.ny_otf == 1) {
     p.otf.mode = 0;
@@ -326,16 +329,21 @@ static int build_plan(GridPlan& p, int gx, int gy, int gz, float dr, float dz, c
   }
   p.g = make_geom(gx, gy, gz);
   int rc;
-  if ((rc = fft_len_init(p.fx, gx))) return rc;
-  if ((rc = fft_len_init(p.fy, gy))) return rc;
-  if ((rc = fft_len_init(p.fz, gz))) return rc;
+  if ((rc = fft_len_init(p.fx, gx, Axis::x))) return rc;
+  if ((rc = fft_len_init(p.fy, gy, Axis::y))) return rc;
+  if ((rc = fft_len_init(p.fz, gz, Axis::z))) return rc;
   return fill_otf(p, dr, dz, o, st);
 }
 
 // Session plan for a decon grid (reused while the grid does not change).
 static int ensure_plan(Session& s, int gx, int gy, int gz) {
   GridPlan& p = s.plan;
-  if (p.valid && p.g.nx == gx && p.g.ny == gy && p.g.nz == gz) return 0;
+  const bool same = p.valid && p.g.nx == gx && p.g.ny == gy && p.g.nz == gz;
+  if (same) {
+    Geom now = p.g;  // the DFT form may have changed the layout since
+    choose_layout(now, p.fx, p.fy);
+    if (now.pair == p.g.pair) return 0;
+  }
   OtfSpec o;
   o.od = s.od;
   o.dkx_otf = s.dkx_otf;
@@ -343,7 +351,13 @@ static int ensure_plan(Session& s, int gx, int gy, int gz) {
   o.dkz_otf = s.dkz_otf;
   o.raw_otf = s.raw_otf.p;
   int rc;
-  if ((rc = build_plan(p, gx, gy, gz, s.dr, s.dz, o, s.stream))) return rc;
+  if (same) {
+    // the OTF table follows the layout (its users on other streams are done)
+    CDX_CHECK(cudaDeviceSynchronize());
+    if ((rc = fill_otf(p, s.dr, s.dz, o, s.stream))) return rc;
+  } else if ((rc = build_plan(p, gx, gy, gz, s.dr, s.dz, o, s.stream))) {
+    return rc;
+  }
   CDX_CHECK(cudaStreamSynchronize(s.stream));
   return 0;
 }
@@ -386,6 +400,7 @@ static int rl_loop(const GridPlan& p, const LoopBufs& b, int nIter, cudaStream_t
   w.partials = b.partials;
   w.lam = b.lam;
   w.max_blocks = b.max_blocks;
+  w.h0 = p.otf.h0;
   const float eps = 1.1920928955078125e-07f;  // std::numeric_limits<float>::epsilon()
   float* X = b.Xa;
   float* Xm1 = b.Xb;
@@ -1570,9 +1585,10 @@ int cdx_rfft3d_device(const float* in, void* out_complex, int nx, int ny, int nz
   FftLen fx, fy, fz;
   DevBuf<float2> S;
   OtfDev none{};
-  int ok = !(fft_len_init(fx, nx) || fft_len_init(fy, ny) || fft_len_init(fz, nz) ||
-             S.ensure((size_t)g.spec_elems()) ||
-             launch_x_fwd(g, fx, in, nullptr, nullptr, 0, S.p, st) ||
+  int ok = !(fft_len_init(fx, nx, Axis::x) || fft_len_init(fy, ny, Axis::y) ||
+             fft_len_init(fz, nz, Axis::z) || S.ensure((size_t)g.spec_elems()));
+  if (ok) choose_layout(g, fx, fy);
+  ok = ok && !(launch_x_fwd(g, fx, in, nullptr, nullptr, 0, S.p, st) ||
              launch_y_pass(g, fy, S.p, false, st) || launch_z_pass(g, fz, S.p, none, false, st, true) ||
              launch_spec_to_std(g, S.p, (float2*)out_complex, st) || cudaStreamSynchronize(st));
   fft_len_free(fx);

@@ -13,8 +13,12 @@
 // folded into the OTF table.  No intermediate real volume is written between
 // the two convolutions.
 #include "decon_common.cuh"
+#include "pair_layout.cuh"
+#include "pair_plans_gen.cuh"
 
 #include <math.h>
+#include <algorithm>
+#include <atomic>
 #include <vector>
 
 namespace cdx {
@@ -28,6 +32,17 @@ Geom make_geom(int nx, int ny, int nz) {
   g.nyp = ny + (ny & 1);
   g.plane = (long long)nz * g.nyp;
   return g;
+}
+
+int sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 152;
+  if ((n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
+    return 152;
+  known[dev].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 // ---------------------------------------------------------------- FFT plans
@@ -84,35 +99,80 @@ static int build_fft_dev(int L, const std::vector<int>& rad, FftDev& d, float2**
       sd = StageDev{1, L, Ns, 0, 1.0f / (float)L, 1.0f / (float)Ns};
     }
   }
-  CDX_CHECK(cudaMalloc(d_tw, sizeof(float2) * L));
-  CDX_CHECK(cudaMemcpy(*d_tw, tw.data(), sizeof(float2) * L, cudaMemcpyHostToDevice));
+  tw.resize(L + (L & 1));  // the paired passes copy it in 16-byte pieces
+  CDX_CHECK(cudaMalloc(d_tw, sizeof(float2) * tw.size()));
+  CDX_CHECK(cudaMemcpy(*d_tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
   d.tw = *d_tw;
   return 0;
 }
 
-int fft_len_init(FftLen& f, int L) {
+// Radices of the paired plan for length L on an axis (empty: none).  y plans of
+// an even height transform points = L / 2 rows in two lanes.
+static std::vector<int> pair_radices(int L, Axis axis, int& points) {
+#define CDX_CASE(LL, N, V, A, B, C)                                                  \
+  case LL:                                                                           \
+    points = N;                                                                      \
+    return B > 1 ? std::vector<int>{A, B, C} : std::vector<int>{A, C};
+  switch (axis) {
+    case Axis::x:
+      switch (L) { CDX_PX_PLANS(CDX_CASE) }
+      break;
+    case Axis::y:
+      switch (L) { CDX_PY_PLANS(CDX_CASE) }
+      break;
+    case Axis::z:
+      switch (L) { CDX_PZ_PLANS(CDX_CASE) }
+      break;
+  }
+#undef CDX_CASE
+  return {};
+}
+
+// Twiddles of a paired plan; with points = L / 2 (y), the factors
+// exp(-2 pi i k / L) of the step across the lanes follow, k < L / 2.
+static int build_pair(FftLen& f, int L, int points, const std::vector<int>& rad) {
+  FftDev d;
+  if (points == L) return build_fft_dev(L, rad, d, &f.d_pair);
+  float2* plan = nullptr;
+  if (int rc = build_fft_dev(points, rad, d, &plan)) return rc;
+  std::vector<float2> w(points);
+  const double two_pi = 6.283185307179586476925286766559;
+  for (int k = 0; k < points; ++k)
+    w[k] = make_float2((float)cos(-two_pi * k / L), (float)sin(-two_pi * k / L));
+  const size_t n = sizeof(float2) * points;
+  cudaError_t e = cudaMalloc(&f.d_pair, 2 * n);
+  if (e == cudaSuccess) e = cudaMemcpy(f.d_pair, plan, n, cudaMemcpyDeviceToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(f.d_pair + points, w.data(), n, cudaMemcpyHostToDevice);
+  cudaFree(plan);
+  if (e != cudaSuccess) set_cuda_error("fft_len_init", e);
+  f.pair_eo = 1;
+  return e;
+}
+
+int fft_len_init(FftLen& f, int L, Axis axis) {
   std::vector<int> rad;
   if (L < 1 || L > kMaxFftLen || !factorize(L, rad)) {
     set_error("fft_len_init", "length is not a product of 2, 3, 5 and 7");
     return cudaErrorInvalidValue;
   }
   if (int rc = build_fft_dev(L, rad, f.dev, &f.d_tw)) return rc;
-  f.has_static = static_radices(L, rad);
-  if (f.has_static) {
-    if (int rc = build_fft_dev(L, rad, f.sdev, &f.d_tws)) return rc;
+  int points = 0;
+  rad = pair_radices(L, axis, points);
+  if (!rad.empty()) {
+    if (int rc = build_pair(f, L, points, rad)) return rc;
   }
-  int pairs = 0;
-  f.has_xr = xr_radices(L, rad, pairs);
-  if (f.has_xr) {
-    if (int rc = build_fft_dev(L, rad, f.xrdev, &f.d_twxr)) return rc;
-  }
-  f.has_gx = gx_radices(L, rad);
-  if (f.has_gx) {
-    if (int rc = build_fft_dev(L, rad, f.gxdev, &f.d_twgx)) return rc;
-  }
-  f.has_gz = gz_radices(L, rad);
-  if (f.has_gz) {
-    if (int rc = build_fft_dev(L, rad, f.gzdev, &f.d_twgz)) return rc;
+  if (axis != Axis::x) {
+    f.has_static = static_radices(L, rad);
+    if (f.has_static) {
+      if (int rc = build_fft_dev(L, rad, f.sdev, &f.d_tws)) return rc;
+    }
+    if (axis == Axis::z) {
+      f.has_gz = gz_radices(L, rad);
+      if (f.has_gz) {
+        if (int rc = build_fft_dev(L, rad, f.gzdev, &f.d_twgz)) return rc;
+      }
+    }
+    return 0;
   }
   int q0 = 0, q1 = 0;
   f.has_tc = tc_plan_radices(L, q0, q1);
@@ -122,6 +182,15 @@ int fft_len_init(FftLen& f, int L) {
     CDX_CHECK(cudaMemset(f.tc.d_err, 0, sizeof(int)));
   }
   return 0;
+}
+
+void choose_layout(Geom& g, const FftLen& fx, const FftLen& fy) {
+  // the generic z pass holds at least one column pair of a tile
+  const bool z_fits = 2 * g.nz <= kMaxThreads * kEpt;
+  // slot offsets within a slice are 32-bit
+  const bool s_fits = (long long)pair_half(g.ny) * 2 * g.nxh < (1LL << 31);
+  g.pair = fx.d_pair && z_fits && s_fits && !(dft_form() == 1 && fx.has_tc);
+  g.eo = g.pair && fy.d_pair && fy.pair_eo;
 }
 
 int tc_check(const FftLen& f) {
@@ -140,56 +209,40 @@ int dft_form() { return g_dft_form; }
 void set_dft_form(int form) { g_dft_form = form; }
 
 void fft_len_free(FftLen& f) {
-  if (f.d_tw) cudaFree(f.d_tw);
-  if (f.d_tws) cudaFree(f.d_tws);
-  if (f.d_twxr) cudaFree(f.d_twxr);
-  if (f.d_twgx) cudaFree(f.d_twgx);
-  f.d_twgx = nullptr;
-  f.gxdev.tw = nullptr;
-  f.has_gx = false;
-  if (f.d_twgz) cudaFree(f.d_twgz);
-  f.d_twgz = nullptr;
-  f.gzdev.tw = nullptr;
-  f.has_gz = false;
-  f.d_tw = nullptr;
-  f.d_tws = nullptr;
-  f.d_twxr = nullptr;
-  f.dev.tw = nullptr;
-  f.sdev.tw = nullptr;
-  f.xrdev.tw = nullptr;
-  f.has_static = false;
-  f.has_xr = false;
+  for (float2** t : {&f.d_tw, &f.d_tws, &f.d_twgz, &f.d_pair}) {
+    if (*t) cudaFree(*t);
+    *t = nullptr;
+  }
+  f.dev.tw = f.sdev.tw = f.gzdev.tw = nullptr;
+  f.has_static = f.has_gz = false;
+  f.pair_eo = 0;
   if (f.has_tc) tc_tables_free(f.tc);
   f.has_tc = false;
 }
 
-// Row pairs per block of the x passes: the registered tile of a compile-time
-// plan, else the generic tile.
-static int x_tile_pairs(int nx) {
+// Pairs per block of the paired x passes.
+static int px_pairs(int nx) {
   switch (nx) {
-#define CDX_PAIRS_CASE(L, PP) \
-  case L:                     \
-    return PP;
-    CDX_X_PLANS(CDX_PAIRS_CASE)
-#undef CDX_PAIRS_CASE
+#define CDX_CASE(LL, N, V, A, B, C) \
+  case LL:                          \
+    return V;
+    CDX_PX_PLANS(CDX_CASE)
+#undef CDX_CASE
     default:
-      return x_pairs(nx);
+      return 1;
   }
 }
 
-// Blocks of the x pass with the most (the smallest tile): the dot-product
+// Most blocks an x pass of the grid launches in either layout: the dot-product
 // partials are sized by it.
 int x_pass_blocks(const Geom& g) {
-  int p = x_tile_pairs(g.nx);
-  std::vector<int> rad;
-  int pxr = 0;
-  if (xr_radices(g.nx, rad, pxr) && pxr < p) p = pxr;
-  int pgx = 0;
-  if (gx_pairs(g.nx, pgx) && pgx < p) p = pgx;
-  return ceil_div(g.ny, 2 * p) * g.nz;
+  const int plain = ceil_div(g.ny, 2 * x_pairs(g.nx));
+  const int pair = ceil_div(pair_half(g.ny), px_pairs(g.nx));
+  return std::max(plain, pair) * g.nz;
 }
 
-__global__ void k_spec_to_std(Geom g, const float2* __restrict__ S, float2* __restrict__ out) {
+__global__ void k_spec_to_std(Geom g, PairGeom pg, const float2* __restrict__ S,
+                              float2* __restrict__ out) {
   const long long n = (long long)g.nz * g.ny * g.nxh;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
@@ -197,12 +250,18 @@ __global__ void k_spec_to_std(Geom g, const float2* __restrict__ S, float2* __re
     const long long r = i / g.nxh;
     const int y = (int)(r % g.ny);
     const int z = (int)(r / g.ny);
-    out[i] = S[(long long)kx * g.plane + (long long)z * g.nyp + y];
+    if (g.pair) {
+      // the paired y pass leaves twice the spectrum
+      const float* p = reinterpret_cast<const float*>(S) + pg.at(kx, z, y);
+      out[i] = make_float2(0.5f * p[0], 0.5f * p[2]);
+    } else {
+      out[i] = S[(long long)kx * g.plane + (long long)z * g.nyp + y];
+    }
   }
 }
 
 int launch_spec_to_std(const Geom& g, const float2* S, float2* out, cudaStream_t st) {
-  k_spec_to_std<<<1216, 256, 0, st>>>(g, S, out);
+  k_spec_to_std<<<1216, 256, 0, st>>>(g, pair_geom(g), S, out);
   CDX_LAUNCH_CHECK("k_spec_to_std");
   return 0;
 }
@@ -256,7 +315,7 @@ int launch_otf_tz(const Geom& g, const float2* raw_otf, const RawOtfDims& od, fl
 // Full 3D (non radially averaged) OTF: trilinear with y/z wrap, as the
 // non-RA branch of dev_otfinterpolate (RLgpuImpl.cu:274-319), laid out in the
 // spectrum order and scaled.
-__global__ void k_otf_full(Geom g, int nxotf, int nyotf, int nzotf, float kxs, float kys, float kzs,
+__global__ void k_otf_full(Geom g, PairGeom pg, int nxotf, int nyotf, int nzotf, float kxs, float kys, float kzs,
                            const float2* __restrict__ otf, float2* __restrict__ full, float scale) {
   const int y = blockIdx.x * blockDim.x + threadIdx.x;
   const int z = blockIdx.y;
@@ -293,13 +352,13 @@ __global__ void k_otf_full(Geom g, int nxotf, int nyotf, int nzotf, float kxs, f
           az * (o100.y * (1 - ay) * (1 - ax) + o101.y * (1 - ay) * ax + o110.y * ay * (1 - ax) +
                 o111.y * ay * ax);
   }
-  full[(long long)kx * g.plane + (long long)z * g.nyp + y] = make_float2(v.x * scale, v.y * scale);
+  st_spec(g, pg, full, kx, z, y, make_float2(v.x * scale, v.y * scale));
 }
 
 int launch_otf_full(const Geom& g, const float2* raw_otf, const RawOtfDims& od, float2* full,
                     float scale, cudaStream_t st) {
   dim3 grid(ceil_div(g.ny, 128), g.nz, g.nxh);
-  k_otf_full<<<grid, 128, 0, st>>>(g, od.nx_otf, od.ny_otf, od.nz_otf, od.kxscale, od.kyscale,
+  k_otf_full<<<grid, 128, 0, st>>>(g, pair_geom(g), od.nx_otf, od.ny_otf, od.nz_otf, od.kxscale, od.kyscale,
                                    od.kzscale, raw_otf, full, scale);
   CDX_LAUNCH_CHECK("k_otf_full");
   return 0;

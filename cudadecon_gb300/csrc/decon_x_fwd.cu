@@ -9,21 +9,11 @@ namespace cdx {
 
 int launch_x_fwd(const Geom& g, const FftLen& fx, const float* X, float* Xm1,
                  const float* lam, int predict, float2* S, cudaStream_t st) {
-  if (fx.has_tc && dft_form() == 1)
+  if (!g.pair && fx.has_tc && dft_form() == 1)
     return launch_xtc_fwd(g, fx.tc, X, Xm1, lam, predict, S, fx.tc.d_err, st);
-  if (fx.has_static) switch (g.nx) {
-#define CDX_CASE(L, PP)                                                                      \
-  case L:                                                                                    \
-    return x_fwd_go<StaticRunner<SP##L, PP, false>>(g, fx.sdev, X, Xm1, lam, predict, S, PP, \
-                                                    splan_threads<SP##L, PP>(), st);
-      CDX_X_PLANS(CDX_CASE)
-#undef CDX_CASE
-      default:
-        break;
-    }
-  if (fx.has_gx) {
+  if (g.pair) {
     bool done = false;
-    const int rc = xgen_fwd(g, fx, X, Xm1, lam, predict, S, st, &done);
+    const int rc = pxgen_fwd(pair_geom(g), fx.d_pair, X, Xm1, lam, predict, S, st, &done);
     if (done || rc) return rc;
   }
   const int P = x_pairs(g.nx);
@@ -68,15 +58,12 @@ static int x_plain_go(const Geom& g, const FftDev& f, const float2* S, float* ou
 
 int launch_x_inv_plain(const Geom& g, const FftLen& fx, const float2* S, float* out,
                        cudaStream_t st) {
-  if (fx.has_static) switch (g.nx) {
-#define CDX_CASE(L, PP) \
-  case L:               \
-    return x_plain_go<StaticRunner<SP##L, PP, false>>(g, fx.sdev, S, out, PP, splan_threads<SP##L, PP>(), st);
-      CDX_X_PLANS(CDX_CASE)
-#undef CDX_CASE
-      default:
-        break;
-    }
+  if (g.pair) {
+    bool done = false;
+    const int rc = pxgen_update(pair_geom(g), fx.d_pair, S, nullptr, out, nullptr, 0, nullptr,
+                                nullptr, 0.f, st, &done);
+    if (done || rc) return rc;
+  }
   const int P = x_pairs(g.nx);
   return x_plain_go<GenericRunner>(g, fx.dev, S, out, P, threads_for((long long)P * g.nx), st);
 }

@@ -1,98 +1,90 @@
-// Generated by cudadecon_gb300/gen_plans.py (do not edit): x-pass kernels
-// of the generated x lengths 140, 200, 288, 384, 500, 648, 810, 1008.
-#include "decon_x_kernels.cuh"
+// Generated by cudadecon_gb300/gen_plans.py (do not edit): paired x-pass kernels
+// of the lengths 135, 245, 400, 625, 882, 1225, 1680.
+#include "decon_px.cuh"
+#include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
 
 namespace cdx {
 
-int xgen_fwd_1(const Geom& g, const FftLen& fx, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_1(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 140:
+    case 135:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX140, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX140, 4>(), st);
-    case 200:
+      return px_fwd_go<PPX135, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 245:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX200, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX200, 4>(), st);
-    case 288:
+      return px_fwd_go<PPX245, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 400:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX288, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX288, 4>(), st);
-    case 384:
+      return px_fwd_go<PPX400, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 625:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX384, 4, false, false, 0, 16, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX384, 4>(), st);
-    case 500:
+      return px_fwd_go<PPX625, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 882:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX500, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX500, 2>(), st);
-    case 648:
+      return px_fwd_go<PPX882, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1225:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX648, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX648, 4>(), st);
-    case 810:
+      return px_fwd_go<PPX1225, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1680:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX810, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX810, 2>(), st);
-    case 1008:
-      *done = true;
-      return x_fwd_go<StaticRunner<SPX1008, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX1008, 2>(), st);
+      return px_fwd_go<PPX1680, 2>(g, tw, X, Xm1, lam, predict, S, st);
     default:
       return 0;
   }
 }
 
-int xgen_ratio_1(const Geom& g, const FftLen& fx, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_1(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 140:
+    case 135:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX140, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX140, 4>(), st);
-    case 200:
+      return px_ratio_go<PPX135, 2>(g, tw, S, raw, eps, st);
+    case 245:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX200, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX200, 4>(), st);
-    case 288:
+      return px_ratio_go<PPX245, 2>(g, tw, S, raw, eps, st);
+    case 400:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX288, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX288, 4>(), st);
-    case 384:
+      return px_ratio_go<PPX400, 2>(g, tw, S, raw, eps, st);
+    case 625:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX384, 4, false, false, 0, 16, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX384, 4>(), st);
-    case 500:
+      return px_ratio_go<PPX625, 2>(g, tw, S, raw, eps, st);
+    case 882:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX500, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX500, 2>(), st);
-    case 648:
+      return px_ratio_go<PPX882, 2>(g, tw, S, raw, eps, st);
+    case 1225:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX648, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX648, 4>(), st);
-    case 810:
+      return px_ratio_go<PPX1225, 2>(g, tw, S, raw, eps, st);
+    case 1680:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX810, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX810, 2>(), st);
-    case 1008:
-      *done = true;
-      return x_ratio_go<StaticRunner<SPX1008, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX1008, 2>(), st);
+      return px_ratio_go<PPX1680, 2>(g, tw, S, raw, eps, st);
     default:
       return 0;
   }
 }
 
-int xgen_update_1(const Geom& g, const FftLen& fx, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork& w, float* lam_next, float eps, cudaStream_t st, bool* done) {
+int pxgen_update_1(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 140:
+    case 135:
       *done = true;
-      return x_update_go<StaticRunner<SPX140, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX140, 4>(), st);
-    case 200:
+      return px_update_go<PPX135, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 245:
       *done = true;
-      return x_update_go<StaticRunner<SPX200, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX200, 4>(), st);
-    case 288:
+      return px_update_go<PPX245, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 400:
       *done = true;
-      return x_update_go<StaticRunner<SPX288, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX288, 4>(), st);
-    case 384:
+      return px_update_go<PPX400, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 625:
       *done = true;
-      return x_update_go<StaticRunner<SPX384, 4, false, false, 0, 16, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX384, 4>(), st);
-    case 500:
+      return px_update_go<PPX625, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 882:
       *done = true;
-      return x_update_go<StaticRunner<SPX500, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX500, 2>(), st);
-    case 648:
+      return px_update_go<PPX882, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1225:
       *done = true;
-      return x_update_go<StaticRunner<SPX648, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX648, 4>(), st);
-    case 810:
+      return px_update_go<PPX1225, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1680:
       *done = true;
-      return x_update_go<StaticRunner<SPX810, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX810, 2>(), st);
-    case 1008:
-      *done = true;
-      return x_update_go<StaticRunner<SPX1008, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX1008, 2>(), st);
+      return px_update_go<PPX1680, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
     default:
       return 0;
   }

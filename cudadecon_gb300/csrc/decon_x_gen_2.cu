@@ -1,89 +1,90 @@
-// Generated by cudadecon_gb300/gen_plans.py (do not edit): x-pass kernels
-// of the generated x lengths 144, 210, 294, 392, 504, 672, 840.
-#include "decon_x_kernels.cuh"
+// Generated by cudadecon_gb300/gen_plans.py (do not edit): paired x-pass kernels
+// of the lengths 140, 250, 405, 630, 896, 1250, 1701.
+#include "decon_px.cuh"
+#include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
 
 namespace cdx {
 
-int xgen_fwd_2(const Geom& g, const FftLen& fx, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_2(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 144:
+    case 140:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX144, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX144, 4>(), st);
-    case 210:
+      return px_fwd_go<PPX140, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 250:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX210, 8, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 8, splan_threads<SPX210, 8>(), st);
-    case 294:
+      return px_fwd_go<PPX250, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 405:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX294, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX294, 4>(), st);
-    case 392:
+      return px_fwd_go<PPX405, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 630:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX392, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX392, 4>(), st);
-    case 504:
+      return px_fwd_go<PPX630, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 896:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX504, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX504, 4>(), st);
-    case 672:
+      return px_fwd_go<PPX896, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1250:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX672, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX672, 4>(), st);
-    case 840:
+      return px_fwd_go<PPX1250, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1701:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX840, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX840, 2>(), st);
+      return px_fwd_go<PPX1701, 2>(g, tw, X, Xm1, lam, predict, S, st);
     default:
       return 0;
   }
 }
 
-int xgen_ratio_2(const Geom& g, const FftLen& fx, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_2(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 144:
+    case 140:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX144, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX144, 4>(), st);
-    case 210:
+      return px_ratio_go<PPX140, 2>(g, tw, S, raw, eps, st);
+    case 250:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX210, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 8, splan_threads<SPX210, 8>(), st);
-    case 294:
+      return px_ratio_go<PPX250, 2>(g, tw, S, raw, eps, st);
+    case 405:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX294, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX294, 4>(), st);
-    case 392:
+      return px_ratio_go<PPX405, 2>(g, tw, S, raw, eps, st);
+    case 630:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX392, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX392, 4>(), st);
-    case 504:
+      return px_ratio_go<PPX630, 2>(g, tw, S, raw, eps, st);
+    case 896:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX504, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX504, 4>(), st);
-    case 672:
+      return px_ratio_go<PPX896, 2>(g, tw, S, raw, eps, st);
+    case 1250:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX672, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX672, 4>(), st);
-    case 840:
+      return px_ratio_go<PPX1250, 2>(g, tw, S, raw, eps, st);
+    case 1701:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX840, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX840, 2>(), st);
+      return px_ratio_go<PPX1701, 2>(g, tw, S, raw, eps, st);
     default:
       return 0;
   }
 }
 
-int xgen_update_2(const Geom& g, const FftLen& fx, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork& w, float* lam_next, float eps, cudaStream_t st, bool* done) {
+int pxgen_update_2(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 144:
+    case 140:
       *done = true;
-      return x_update_go<StaticRunner<SPX144, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX144, 4>(), st);
-    case 210:
+      return px_update_go<PPX140, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 250:
       *done = true;
-      return x_update_go<StaticRunner<SPX210, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 8, splan_threads<SPX210, 8>(), st);
-    case 294:
+      return px_update_go<PPX250, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 405:
       *done = true;
-      return x_update_go<StaticRunner<SPX294, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX294, 4>(), st);
-    case 392:
+      return px_update_go<PPX405, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 630:
       *done = true;
-      return x_update_go<StaticRunner<SPX392, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX392, 4>(), st);
-    case 504:
+      return px_update_go<PPX630, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 896:
       *done = true;
-      return x_update_go<StaticRunner<SPX504, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX504, 4>(), st);
-    case 672:
+      return px_update_go<PPX896, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1250:
       *done = true;
-      return x_update_go<StaticRunner<SPX672, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX672, 4>(), st);
-    case 840:
+      return px_update_go<PPX1250, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1701:
       *done = true;
-      return x_update_go<StaticRunner<SPX840, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX840, 2>(), st);
+      return px_update_go<PPX1701, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
     default:
       return 0;
   }

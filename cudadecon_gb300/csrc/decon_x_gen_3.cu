@@ -1,89 +1,90 @@
-// Generated by cudadecon_gb300/gen_plans.py (do not edit): x-pass kernels
-// of the generated x lengths 147, 216, 300, 400, 525, 675, 864.
-#include "decon_x_kernels.cuh"
+// Generated by cudadecon_gb300/gen_plans.py (do not edit): paired x-pass kernels
+// of the lengths 144, 252, 420, 640, 900, 1260, 1728.
+#include "decon_px.cuh"
+#include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
 
 namespace cdx {
 
-int xgen_fwd_3(const Geom& g, const FftLen& fx, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_3(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 147:
+    case 144:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX147, 8, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 8, splan_threads<SPX147, 8>(), st);
-    case 216:
+      return px_fwd_go<PPX144, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 252:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX216, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX216, 4>(), st);
-    case 300:
+      return px_fwd_go<PPX252, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 420:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX300, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX300, 4>(), st);
-    case 400:
+      return px_fwd_go<PPX420, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 640:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX400, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX400, 4>(), st);
-    case 525:
+      return px_fwd_go<PPX640, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 900:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX525, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX525, 2>(), st);
-    case 675:
+      return px_fwd_go<PPX900, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1260:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX675, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX675, 2>(), st);
-    case 864:
+      return px_fwd_go<PPX1260, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1728:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX864, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX864, 2>(), st);
+      return px_fwd_go<PPX1728, 2>(g, tw, X, Xm1, lam, predict, S, st);
     default:
       return 0;
   }
 }
 
-int xgen_ratio_3(const Geom& g, const FftLen& fx, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_3(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 147:
+    case 144:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX147, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 8, splan_threads<SPX147, 8>(), st);
-    case 216:
+      return px_ratio_go<PPX144, 2>(g, tw, S, raw, eps, st);
+    case 252:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX216, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX216, 4>(), st);
-    case 300:
+      return px_ratio_go<PPX252, 2>(g, tw, S, raw, eps, st);
+    case 420:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX300, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX300, 4>(), st);
-    case 400:
+      return px_ratio_go<PPX420, 2>(g, tw, S, raw, eps, st);
+    case 640:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX400, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX400, 4>(), st);
-    case 525:
+      return px_ratio_go<PPX640, 2>(g, tw, S, raw, eps, st);
+    case 900:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX525, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX525, 2>(), st);
-    case 675:
+      return px_ratio_go<PPX900, 2>(g, tw, S, raw, eps, st);
+    case 1260:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX675, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX675, 2>(), st);
-    case 864:
+      return px_ratio_go<PPX1260, 2>(g, tw, S, raw, eps, st);
+    case 1728:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX864, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX864, 2>(), st);
+      return px_ratio_go<PPX1728, 2>(g, tw, S, raw, eps, st);
     default:
       return 0;
   }
 }
 
-int xgen_update_3(const Geom& g, const FftLen& fx, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork& w, float* lam_next, float eps, cudaStream_t st, bool* done) {
+int pxgen_update_3(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 147:
+    case 144:
       *done = true;
-      return x_update_go<StaticRunner<SPX147, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 8, splan_threads<SPX147, 8>(), st);
-    case 216:
+      return px_update_go<PPX144, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 252:
       *done = true;
-      return x_update_go<StaticRunner<SPX216, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX216, 4>(), st);
-    case 300:
+      return px_update_go<PPX252, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 420:
       *done = true;
-      return x_update_go<StaticRunner<SPX300, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX300, 4>(), st);
-    case 400:
+      return px_update_go<PPX420, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 640:
       *done = true;
-      return x_update_go<StaticRunner<SPX400, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX400, 4>(), st);
-    case 525:
+      return px_update_go<PPX640, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 900:
       *done = true;
-      return x_update_go<StaticRunner<SPX525, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX525, 2>(), st);
-    case 675:
+      return px_update_go<PPX900, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1260:
       *done = true;
-      return x_update_go<StaticRunner<SPX675, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX675, 2>(), st);
-    case 864:
+      return px_update_go<PPX1260, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1728:
       *done = true;
-      return x_update_go<StaticRunner<SPX864, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX864, 2>(), st);
+      return px_update_go<PPX1728, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
     default:
       return 0;
   }

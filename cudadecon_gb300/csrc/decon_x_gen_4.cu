@@ -1,89 +1,90 @@
-// Generated by cudadecon_gb300/gen_plans.py (do not edit): x-pass kernels
-// of the generated x lengths 150, 224, 315, 405, 540, 686, 875.
-#include "decon_x_kernels.cuh"
+// Generated by cudadecon_gb300/gen_plans.py (do not edit): paired x-pass kernels
+// of the lengths 147, 256, 432, 648, 945, 1280, 1750.
+#include "decon_px.cuh"
+#include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
 
 namespace cdx {
 
-int xgen_fwd_4(const Geom& g, const FftLen& fx, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_4(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 150:
+    case 147:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX150, 8, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 8, splan_threads<SPX150, 8>(), st);
-    case 224:
+      return px_fwd_go<PPX147, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 256:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX224, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX224, 4>(), st);
-    case 315:
+      return px_fwd_go<PPX256, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 432:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX315, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX315, 4>(), st);
-    case 405:
+      return px_fwd_go<PPX432, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 648:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX405, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX405, 4>(), st);
-    case 540:
+      return px_fwd_go<PPX648, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 945:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX540, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX540, 4>(), st);
-    case 686:
+      return px_fwd_go<PPX945, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1280:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX686, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX686, 4>(), st);
-    case 875:
+      return px_fwd_go<PPX1280, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1750:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX875, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX875, 2>(), st);
+      return px_fwd_go<PPX1750, 2>(g, tw, X, Xm1, lam, predict, S, st);
     default:
       return 0;
   }
 }
 
-int xgen_ratio_4(const Geom& g, const FftLen& fx, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_4(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 150:
+    case 147:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX150, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 8, splan_threads<SPX150, 8>(), st);
-    case 224:
+      return px_ratio_go<PPX147, 2>(g, tw, S, raw, eps, st);
+    case 256:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX224, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX224, 4>(), st);
-    case 315:
+      return px_ratio_go<PPX256, 2>(g, tw, S, raw, eps, st);
+    case 432:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX315, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX315, 4>(), st);
-    case 405:
+      return px_ratio_go<PPX432, 2>(g, tw, S, raw, eps, st);
+    case 648:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX405, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX405, 4>(), st);
-    case 540:
+      return px_ratio_go<PPX648, 2>(g, tw, S, raw, eps, st);
+    case 945:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX540, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX540, 4>(), st);
-    case 686:
+      return px_ratio_go<PPX945, 2>(g, tw, S, raw, eps, st);
+    case 1280:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX686, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX686, 4>(), st);
-    case 875:
+      return px_ratio_go<PPX1280, 2>(g, tw, S, raw, eps, st);
+    case 1750:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX875, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX875, 2>(), st);
+      return px_ratio_go<PPX1750, 2>(g, tw, S, raw, eps, st);
     default:
       return 0;
   }
 }
 
-int xgen_update_4(const Geom& g, const FftLen& fx, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork& w, float* lam_next, float eps, cudaStream_t st, bool* done) {
+int pxgen_update_4(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 150:
+    case 147:
       *done = true;
-      return x_update_go<StaticRunner<SPX150, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 8, splan_threads<SPX150, 8>(), st);
-    case 224:
+      return px_update_go<PPX147, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 256:
       *done = true;
-      return x_update_go<StaticRunner<SPX224, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX224, 4>(), st);
-    case 315:
+      return px_update_go<PPX256, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 432:
       *done = true;
-      return x_update_go<StaticRunner<SPX315, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX315, 4>(), st);
-    case 405:
+      return px_update_go<PPX432, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 648:
       *done = true;
-      return x_update_go<StaticRunner<SPX405, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX405, 4>(), st);
-    case 540:
+      return px_update_go<PPX648, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 945:
       *done = true;
-      return x_update_go<StaticRunner<SPX540, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX540, 4>(), st);
-    case 686:
+      return px_update_go<PPX945, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1280:
       *done = true;
-      return x_update_go<StaticRunner<SPX686, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX686, 4>(), st);
-    case 875:
+      return px_update_go<PPX1280, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1750:
       *done = true;
-      return x_update_go<StaticRunner<SPX875, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX875, 2>(), st);
+      return px_update_go<PPX1750, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
     default:
       return 0;
   }

@@ -1,89 +1,90 @@
-// Generated by cudadecon_gb300/gen_plans.py (do not edit): x-pass kernels
-// of the generated x lengths 160, 225, 320, 420, 560, 700, 882.
-#include "decon_x_kernels.cuh"
+// Generated by cudadecon_gb300/gen_plans.py (do not edit): paired x-pass kernels
+// of the lengths 150, 270, 441, 672, 960, 1296, 1764.
+#include "decon_px.cuh"
+#include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
 
 namespace cdx {
 
-int xgen_fwd_5(const Geom& g, const FftLen& fx, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_5(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 160:
+    case 150:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX160, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX160, 4>(), st);
-    case 225:
+      return px_fwd_go<PPX150, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 270:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX225, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX225, 2>(), st);
-    case 320:
+      return px_fwd_go<PPX270, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 441:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX320, 4, false, false, 0, 16, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX320, 4>(), st);
-    case 420:
+      return px_fwd_go<PPX441, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 672:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX420, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX420, 4>(), st);
-    case 560:
+      return px_fwd_go<PPX672, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 960:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX560, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX560, 4>(), st);
-    case 700:
+      return px_fwd_go<PPX960, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1296:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX700, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX700, 4>(), st);
-    case 882:
+      return px_fwd_go<PPX1296, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1764:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX882, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX882, 2>(), st);
+      return px_fwd_go<PPX1764, 2>(g, tw, X, Xm1, lam, predict, S, st);
     default:
       return 0;
   }
 }
 
-int xgen_ratio_5(const Geom& g, const FftLen& fx, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_5(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 160:
+    case 150:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX160, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX160, 4>(), st);
-    case 225:
+      return px_ratio_go<PPX150, 2>(g, tw, S, raw, eps, st);
+    case 270:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX225, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX225, 2>(), st);
-    case 320:
+      return px_ratio_go<PPX270, 2>(g, tw, S, raw, eps, st);
+    case 441:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX320, 4, false, false, 0, 16, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX320, 4>(), st);
-    case 420:
+      return px_ratio_go<PPX441, 2>(g, tw, S, raw, eps, st);
+    case 672:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX420, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX420, 4>(), st);
-    case 560:
+      return px_ratio_go<PPX672, 2>(g, tw, S, raw, eps, st);
+    case 960:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX560, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX560, 4>(), st);
-    case 700:
+      return px_ratio_go<PPX960, 2>(g, tw, S, raw, eps, st);
+    case 1296:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX700, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX700, 4>(), st);
-    case 882:
+      return px_ratio_go<PPX1296, 2>(g, tw, S, raw, eps, st);
+    case 1764:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX882, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX882, 2>(), st);
+      return px_ratio_go<PPX1764, 2>(g, tw, S, raw, eps, st);
     default:
       return 0;
   }
 }
 
-int xgen_update_5(const Geom& g, const FftLen& fx, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork& w, float* lam_next, float eps, cudaStream_t st, bool* done) {
+int pxgen_update_5(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 160:
+    case 150:
       *done = true;
-      return x_update_go<StaticRunner<SPX160, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX160, 4>(), st);
-    case 225:
+      return px_update_go<PPX150, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 270:
       *done = true;
-      return x_update_go<StaticRunner<SPX225, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX225, 2>(), st);
-    case 320:
+      return px_update_go<PPX270, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 441:
       *done = true;
-      return x_update_go<StaticRunner<SPX320, 4, false, false, 0, 16, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX320, 4>(), st);
-    case 420:
+      return px_update_go<PPX441, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 672:
       *done = true;
-      return x_update_go<StaticRunner<SPX420, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX420, 4>(), st);
-    case 560:
+      return px_update_go<PPX672, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 960:
       *done = true;
-      return x_update_go<StaticRunner<SPX560, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX560, 4>(), st);
-    case 700:
+      return px_update_go<PPX960, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1296:
       *done = true;
-      return x_update_go<StaticRunner<SPX700, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX700, 4>(), st);
-    case 882:
+      return px_update_go<PPX1296, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1764:
       *done = true;
-      return x_update_go<StaticRunner<SPX882, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX882, 2>(), st);
+      return px_update_go<PPX1764, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
     default:
       return 0;
   }

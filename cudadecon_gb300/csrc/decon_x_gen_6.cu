@@ -1,89 +1,90 @@
-// Generated by cudadecon_gb300/gen_plans.py (do not edit): x-pass kernels
-// of the generated x lengths 162, 240, 324, 432, 567, 720, 896.
-#include "decon_x_kernels.cuh"
+// Generated by cudadecon_gb300/gen_plans.py (do not edit): paired x-pass kernels
+// of the lengths 160, 280, 448, 675, 972, 1323, 1792.
+#include "decon_px.cuh"
+#include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
 
 namespace cdx {
 
-int xgen_fwd_6(const Geom& g, const FftLen& fx, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_6(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 162:
+    case 160:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX162, 8, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 8, splan_threads<SPX162, 8>(), st);
-    case 240:
+      return px_fwd_go<PPX160, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 280:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX240, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX240, 4>(), st);
-    case 324:
+      return px_fwd_go<PPX280, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 448:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX324, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX324, 4>(), st);
-    case 432:
+      return px_fwd_go<PPX448, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 675:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX432, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX432, 4>(), st);
-    case 567:
+      return px_fwd_go<PPX675, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 972:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX567, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX567, 2>(), st);
-    case 720:
+      return px_fwd_go<PPX972, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1323:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX720, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX720, 2>(), st);
-    case 896:
+      return px_fwd_go<PPX1323, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1792:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX896, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX896, 2>(), st);
+      return px_fwd_go<PPX1792, 2>(g, tw, X, Xm1, lam, predict, S, st);
     default:
       return 0;
   }
 }
 
-int xgen_ratio_6(const Geom& g, const FftLen& fx, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_6(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 162:
+    case 160:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX162, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 8, splan_threads<SPX162, 8>(), st);
-    case 240:
+      return px_ratio_go<PPX160, 2>(g, tw, S, raw, eps, st);
+    case 280:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX240, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX240, 4>(), st);
-    case 324:
+      return px_ratio_go<PPX280, 2>(g, tw, S, raw, eps, st);
+    case 448:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX324, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX324, 4>(), st);
-    case 432:
+      return px_ratio_go<PPX448, 2>(g, tw, S, raw, eps, st);
+    case 675:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX432, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX432, 4>(), st);
-    case 567:
+      return px_ratio_go<PPX675, 2>(g, tw, S, raw, eps, st);
+    case 972:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX567, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX567, 2>(), st);
-    case 720:
+      return px_ratio_go<PPX972, 2>(g, tw, S, raw, eps, st);
+    case 1323:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX720, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX720, 2>(), st);
-    case 896:
+      return px_ratio_go<PPX1323, 2>(g, tw, S, raw, eps, st);
+    case 1792:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX896, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX896, 2>(), st);
+      return px_ratio_go<PPX1792, 2>(g, tw, S, raw, eps, st);
     default:
       return 0;
   }
 }
 
-int xgen_update_6(const Geom& g, const FftLen& fx, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork& w, float* lam_next, float eps, cudaStream_t st, bool* done) {
+int pxgen_update_6(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 162:
+    case 160:
       *done = true;
-      return x_update_go<StaticRunner<SPX162, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 8, splan_threads<SPX162, 8>(), st);
-    case 240:
+      return px_update_go<PPX160, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 280:
       *done = true;
-      return x_update_go<StaticRunner<SPX240, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX240, 4>(), st);
-    case 324:
+      return px_update_go<PPX280, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 448:
       *done = true;
-      return x_update_go<StaticRunner<SPX324, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX324, 4>(), st);
-    case 432:
+      return px_update_go<PPX448, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 675:
       *done = true;
-      return x_update_go<StaticRunner<SPX432, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX432, 4>(), st);
-    case 567:
+      return px_update_go<PPX675, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 972:
       *done = true;
-      return x_update_go<StaticRunner<SPX567, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX567, 2>(), st);
-    case 720:
+      return px_update_go<PPX972, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1323:
       *done = true;
-      return x_update_go<StaticRunner<SPX720, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX720, 2>(), st);
-    case 896:
+      return px_update_go<PPX1323, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1792:
       *done = true;
-      return x_update_go<StaticRunner<SPX896, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX896, 2>(), st);
+      return px_update_go<PPX1792, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
     default:
       return 0;
   }

@@ -1,89 +1,90 @@
-// Generated by cudadecon_gb300/gen_plans.py (do not edit): x-pass kernels
-// of the generated x lengths 168, 243, 336, 441, 576, 729, 900.
-#include "decon_x_kernels.cuh"
+// Generated by cudadecon_gb300/gen_plans.py (do not edit): paired x-pass kernels
+// of the lengths 162, 288, 450, 686, 980, 1344, 1800.
+#include "decon_px.cuh"
+#include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
 
 namespace cdx {
 
-int xgen_fwd_7(const Geom& g, const FftLen& fx, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_7(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 168:
+    case 162:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX168, 8, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 8, splan_threads<SPX168, 8>(), st);
-    case 243:
+      return px_fwd_go<PPX162, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 288:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX243, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX243, 4>(), st);
-    case 336:
+      return px_fwd_go<PPX288, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 450:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX336, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX336, 4>(), st);
-    case 441:
+      return px_fwd_go<PPX450, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 686:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX441, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX441, 4>(), st);
-    case 576:
+      return px_fwd_go<PPX686, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 980:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX576, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX576, 2>(), st);
-    case 729:
+      return px_fwd_go<PPX980, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1344:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX729, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX729, 4>(), st);
-    case 900:
+      return px_fwd_go<PPX1344, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1800:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX900, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX900, 2>(), st);
+      return px_fwd_go<PPX1800, 2>(g, tw, X, Xm1, lam, predict, S, st);
     default:
       return 0;
   }
 }
 
-int xgen_ratio_7(const Geom& g, const FftLen& fx, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_7(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 168:
+    case 162:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX168, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 8, splan_threads<SPX168, 8>(), st);
-    case 243:
+      return px_ratio_go<PPX162, 2>(g, tw, S, raw, eps, st);
+    case 288:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX243, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX243, 4>(), st);
-    case 336:
+      return px_ratio_go<PPX288, 2>(g, tw, S, raw, eps, st);
+    case 450:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX336, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX336, 4>(), st);
-    case 441:
+      return px_ratio_go<PPX450, 2>(g, tw, S, raw, eps, st);
+    case 686:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX441, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX441, 4>(), st);
-    case 576:
+      return px_ratio_go<PPX686, 2>(g, tw, S, raw, eps, st);
+    case 980:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX576, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX576, 2>(), st);
-    case 729:
+      return px_ratio_go<PPX980, 2>(g, tw, S, raw, eps, st);
+    case 1344:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX729, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX729, 4>(), st);
-    case 900:
+      return px_ratio_go<PPX1344, 2>(g, tw, S, raw, eps, st);
+    case 1800:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX900, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX900, 2>(), st);
+      return px_ratio_go<PPX1800, 2>(g, tw, S, raw, eps, st);
     default:
       return 0;
   }
 }
 
-int xgen_update_7(const Geom& g, const FftLen& fx, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork& w, float* lam_next, float eps, cudaStream_t st, bool* done) {
+int pxgen_update_7(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 168:
+    case 162:
       *done = true;
-      return x_update_go<StaticRunner<SPX168, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 8, splan_threads<SPX168, 8>(), st);
-    case 243:
+      return px_update_go<PPX162, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 288:
       *done = true;
-      return x_update_go<StaticRunner<SPX243, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX243, 4>(), st);
-    case 336:
+      return px_update_go<PPX288, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 450:
       *done = true;
-      return x_update_go<StaticRunner<SPX336, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX336, 4>(), st);
-    case 441:
+      return px_update_go<PPX450, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 686:
       *done = true;
-      return x_update_go<StaticRunner<SPX441, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX441, 4>(), st);
-    case 576:
+      return px_update_go<PPX686, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 980:
       *done = true;
-      return x_update_go<StaticRunner<SPX576, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX576, 2>(), st);
-    case 729:
+      return px_update_go<PPX980, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1344:
       *done = true;
-      return x_update_go<StaticRunner<SPX729, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX729, 4>(), st);
-    case 900:
+      return px_update_go<PPX1344, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1800:
       *done = true;
-      return x_update_go<StaticRunner<SPX900, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX900, 2>(), st);
+      return px_update_go<PPX1800, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
     default:
       return 0;
   }

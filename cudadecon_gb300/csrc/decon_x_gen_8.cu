@@ -1,89 +1,90 @@
-// Generated by cudadecon_gb300/gen_plans.py (do not edit): x-pass kernels
-// of the generated x lengths 175, 245, 343, 448, 588, 735, 945.
-#include "decon_x_kernels.cuh"
+// Generated by cudadecon_gb300/gen_plans.py (do not edit): paired x-pass kernels
+// of the lengths 168, 294, 480, 700, 1000, 1350, 1875.
+#include "decon_px.cuh"
+#include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
 
 namespace cdx {
 
-int xgen_fwd_8(const Geom& g, const FftLen& fx, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_8(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 175:
+    case 168:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX175, 8, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 8, splan_threads<SPX175, 8>(), st);
-    case 245:
+      return px_fwd_go<PPX168, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 294:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX245, 8, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 8, splan_threads<SPX245, 8>(), st);
-    case 343:
+      return px_fwd_go<PPX294, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 480:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX343, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX343, 4>(), st);
-    case 448:
+      return px_fwd_go<PPX480, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 700:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX448, 4, false, false, 0, 16, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX448, 4>(), st);
-    case 588:
+      return px_fwd_go<PPX700, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1000:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX588, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX588, 4>(), st);
-    case 735:
+      return px_fwd_go<PPX1000, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1350:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX735, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX735, 2>(), st);
-    case 945:
+      return px_fwd_go<PPX1350, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1875:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX945, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX945, 2>(), st);
+      return px_fwd_go<PPX1875, 2>(g, tw, X, Xm1, lam, predict, S, st);
     default:
       return 0;
   }
 }
 
-int xgen_ratio_8(const Geom& g, const FftLen& fx, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_8(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 175:
+    case 168:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX175, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 8, splan_threads<SPX175, 8>(), st);
-    case 245:
+      return px_ratio_go<PPX168, 2>(g, tw, S, raw, eps, st);
+    case 294:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX245, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 8, splan_threads<SPX245, 8>(), st);
-    case 343:
+      return px_ratio_go<PPX294, 2>(g, tw, S, raw, eps, st);
+    case 480:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX343, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX343, 4>(), st);
-    case 448:
+      return px_ratio_go<PPX480, 2>(g, tw, S, raw, eps, st);
+    case 700:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX448, 4, false, false, 0, 16, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX448, 4>(), st);
-    case 588:
+      return px_ratio_go<PPX700, 2>(g, tw, S, raw, eps, st);
+    case 1000:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX588, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX588, 4>(), st);
-    case 735:
+      return px_ratio_go<PPX1000, 2>(g, tw, S, raw, eps, st);
+    case 1350:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX735, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX735, 2>(), st);
-    case 945:
+      return px_ratio_go<PPX1350, 2>(g, tw, S, raw, eps, st);
+    case 1875:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX945, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX945, 2>(), st);
+      return px_ratio_go<PPX1875, 2>(g, tw, S, raw, eps, st);
     default:
       return 0;
   }
 }
 
-int xgen_update_8(const Geom& g, const FftLen& fx, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork& w, float* lam_next, float eps, cudaStream_t st, bool* done) {
+int pxgen_update_8(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 175:
+    case 168:
       *done = true;
-      return x_update_go<StaticRunner<SPX175, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 8, splan_threads<SPX175, 8>(), st);
-    case 245:
+      return px_update_go<PPX168, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 294:
       *done = true;
-      return x_update_go<StaticRunner<SPX245, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 8, splan_threads<SPX245, 8>(), st);
-    case 343:
+      return px_update_go<PPX294, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 480:
       *done = true;
-      return x_update_go<StaticRunner<SPX343, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX343, 4>(), st);
-    case 448:
+      return px_update_go<PPX480, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 700:
       *done = true;
-      return x_update_go<StaticRunner<SPX448, 4, false, false, 0, 16, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX448, 4>(), st);
-    case 588:
+      return px_update_go<PPX700, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1000:
       *done = true;
-      return x_update_go<StaticRunner<SPX588, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX588, 4>(), st);
-    case 735:
+      return px_update_go<PPX1000, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1350:
       *done = true;
-      return x_update_go<StaticRunner<SPX735, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX735, 2>(), st);
-    case 945:
+      return px_update_go<PPX1350, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1875:
       *done = true;
-      return x_update_go<StaticRunner<SPX945, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX945, 2>(), st);
+      return px_update_go<PPX1875, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
     default:
       return 0;
   }

@@ -1,89 +1,90 @@
-// Generated by cudadecon_gb300/gen_plans.py (do not edit): x-pass kernels
-// of the generated x lengths 180, 250, 350, 450, 600, 750, 960.
-#include "decon_x_kernels.cuh"
+// Generated by cudadecon_gb300/gen_plans.py (do not edit): paired x-pass kernels
+// of the lengths 175, 300, 486, 720, 1008, 1372, 1890.
+#include "decon_px.cuh"
+#include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
 
 namespace cdx {
 
-int xgen_fwd_9(const Geom& g, const FftLen& fx, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_9(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 180:
+    case 175:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX180, 8, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 8, splan_threads<SPX180, 8>(), st);
-    case 250:
+      return px_fwd_go<PPX175, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 300:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX250, 8, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 8, splan_threads<SPX250, 8>(), st);
-    case 350:
+      return px_fwd_go<PPX300, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 486:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX350, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX350, 4>(), st);
-    case 450:
+      return px_fwd_go<PPX486, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 720:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX450, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX450, 4>(), st);
-    case 600:
+      return px_fwd_go<PPX720, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1008:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX600, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX600, 2>(), st);
-    case 750:
+      return px_fwd_go<PPX1008, 2>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1372:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX750, 4, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 4, splan_threads<SPX750, 4>(), st);
-    case 960:
+      return px_fwd_go<PPX1372, 4>(g, tw, X, Xm1, lam, predict, S, st);
+    case 1890:
       *done = true;
-      return x_fwd_go<StaticRunner<SPX960, 2, false, false, 0, 0, 0>>(g, fx.gxdev, X, Xm1, lam, predict, S, 2, splan_threads<SPX960, 2>(), st);
+      return px_fwd_go<PPX1890, 2>(g, tw, X, Xm1, lam, predict, S, st);
     default:
       return 0;
   }
 }
 
-int xgen_ratio_9(const Geom& g, const FftLen& fx, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_9(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 180:
+    case 175:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX180, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 8, splan_threads<SPX180, 8>(), st);
-    case 250:
+      return px_ratio_go<PPX175, 2>(g, tw, S, raw, eps, st);
+    case 300:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX250, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 8, splan_threads<SPX250, 8>(), st);
-    case 350:
+      return px_ratio_go<PPX300, 2>(g, tw, S, raw, eps, st);
+    case 486:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX350, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX350, 4>(), st);
-    case 450:
+      return px_ratio_go<PPX486, 2>(g, tw, S, raw, eps, st);
+    case 720:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX450, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX450, 4>(), st);
-    case 600:
+      return px_ratio_go<PPX720, 2>(g, tw, S, raw, eps, st);
+    case 1008:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX600, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX600, 2>(), st);
-    case 750:
+      return px_ratio_go<PPX1008, 2>(g, tw, S, raw, eps, st);
+    case 1372:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX750, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 4, splan_threads<SPX750, 4>(), st);
-    case 960:
+      return px_ratio_go<PPX1372, 4>(g, tw, S, raw, eps, st);
+    case 1890:
       *done = true;
-      return x_ratio_go<StaticRunner<SPX960, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, raw, eps, 2, splan_threads<SPX960, 2>(), st);
+      return px_ratio_go<PPX1890, 2>(g, tw, S, raw, eps, st);
     default:
       return 0;
   }
 }
 
-int xgen_update_9(const Geom& g, const FftLen& fx, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork& w, float* lam_next, float eps, cudaStream_t st, bool* done) {
+int pxgen_update_9(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
-    case 180:
+    case 175:
       *done = true;
-      return x_update_go<StaticRunner<SPX180, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 8, splan_threads<SPX180, 8>(), st);
-    case 250:
+      return px_update_go<PPX175, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 300:
       *done = true;
-      return x_update_go<StaticRunner<SPX250, 8, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 8, splan_threads<SPX250, 8>(), st);
-    case 350:
+      return px_update_go<PPX300, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 486:
       *done = true;
-      return x_update_go<StaticRunner<SPX350, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX350, 4>(), st);
-    case 450:
+      return px_update_go<PPX486, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 720:
       *done = true;
-      return x_update_go<StaticRunner<SPX450, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX450, 4>(), st);
-    case 600:
+      return px_update_go<PPX720, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1008:
       *done = true;
-      return x_update_go<StaticRunner<SPX600, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX600, 2>(), st);
-    case 750:
+      return px_update_go<PPX1008, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1372:
       *done = true;
-      return x_update_go<StaticRunner<SPX750, 4, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 4, splan_threads<SPX750, 4>(), st);
-    case 960:
+      return px_update_go<PPX1372, 4>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+    case 1890:
       *done = true;
-      return x_update_go<StaticRunner<SPX960, 2, false, false, 0, 0, 0>>(g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, 2, splan_threads<SPX960, 2>(), st);
+      return px_update_go<PPX1890, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
     default:
       return 0;
   }

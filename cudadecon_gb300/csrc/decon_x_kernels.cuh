@@ -1,10 +1,7 @@
-// The x-pass kernels of the plain form as templates over the transform
-// runner (compile-time plan or generic engine) with their launch helpers:
-// forward x pass with the prediction prologue, inverse x pass with the RL
-// ratio and the forward transform of the ratio, inverse x pass with the
-// estimate update and the dot products.  decon_x_fwd.cu, decon_x_ratio.cu and
-// decon_x_update.cu dispatch the registered lengths; the generated units
-// decon_x_gen_*.cu instantiate the generated plans.
+// The x-pass kernels on the generic engine (lengths without a paired plan, see
+// decon_px.cuh) with their launch helpers: forward x pass with the prediction
+// prologue, inverse x pass with the RL ratio and the forward transform of the
+// ratio, inverse x pass with the estimate update and the dot products.
 #pragma once
 
 #include <algorithm>
@@ -87,13 +84,8 @@ k_x_inv_ratio_fwd(Geom g, FftDev fx, float2* __restrict__ S, const float* __rest
   cp_async_wait_all();
   __syncthreads();
   const RatioStore<typename Run::Tile> rs{io, raws, y0, g.ny, nx, eps};
-  if constexpr (Run::kStatic) {
-    const PackedSpecLoadS<Run::SPlanT::kL> ld{stg, (nr + 1) / 2};
-    Run::template run<true>(fx, P, 1.f, false, stw, io, ld, rs);
-  } else {
-    const PackedSpecLoad ld{stg, g.nxh, nx, (nr + 1) / 2};
-    Run::template run<true>(fx, P, 1.f, false, stw, io, ld, rs);
-  }
+  const PackedSpecLoad ld{stg, g.nxh, nx, (nr + 1) / 2};
+  Run::template run<true>(fx, P, 1.f, false, stw, io, ld, rs);
   Run::template run<false>(fx, P, 1.f, false, stw, io, io, io);
   store_half_spectra<Run::kV>(g, io, P, z, y0, S);
 }
@@ -192,13 +184,8 @@ k_x_inv_update(Geom g, FftDev fx, const float2* __restrict__ S, const float* Y, 
   __syncthreads();
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   const UpdateStore us{Ys, Gs, Xout, G, dots, (long long)z * g.ny * nx, y0, g.ny, nx, acc};
-  if constexpr (Run::kStatic) {
-    const PackedSpecLoadS<Run::SPlanT::kL> ld{stg, (nr + 1) / 2};
-    Run::template run<true>(fx, P, 1.f, false, stw, io, ld, us);
-  } else {
-    const PackedSpecLoad ld{stg, g.nxh, nx, (nr + 1) / 2};
-    Run::template run<true>(fx, P, 1.f, false, stw, io, ld, us);
-  }
+  const PackedSpecLoad ld{stg, g.nxh, nx, (nr + 1) / 2};
+  Run::template run<true>(fx, P, 1.f, false, stw, io, ld, us);
   if (!dots) return;
   const float4 sum = block_sum2_ff(acc[0], acc[1], acc[2], acc[3], red);
   if (threadIdx.x == 0) partials[blockIdx.y * gridDim.x + blockIdx.x] = sum;

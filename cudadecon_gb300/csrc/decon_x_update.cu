@@ -49,35 +49,14 @@ int launch_lambda(const float4* partials, int nblk, float* lam_next, float eps, 
 int launch_x_inv_update(const Geom& g, const FftLen& fx, const float2* S, const float* Y,
                         float* Xout, float* G, int dots, RLWork& w, float* lam_next, float eps,
                         cudaStream_t st) {
-  if (fx.has_tc && dft_form() == 1)
-    return launch_xtc_update(g, fx.tc, S, Y, Xout, G, dots, w, lam_next, eps, fx.tc.d_err, st);
-  if (fx.has_xr) switch (g.nx) {
-#define CDX_XR_CASE(L, PP, ...)                                                                 \
-  case L:                                                                                       \
-    return x_update_go<StaticRunner<SPR##L, PP, false>>(g, fx.xrdev, S, Y, Xout, G, dots, w,    \
-                                                        lam_next, eps, PP,                      \
-                                                        splan_threads<SPR##L, PP>(), st);
-      CDX_XR_PLANS(CDX_XR_CASE)
-#undef CDX_XR_CASE
-      default:
-        break;
-    }
-  if (fx.has_static) switch (g.nx) {
-#define CDX_CASE(L, PP)                                                                    \
-  case L:                                                                                  \
-    return x_update_go<StaticRunner<SP##L, PP, false>>(g, fx.sdev, S, Y, Xout, G, dots, \
-                                                              w, lam_next, eps, PP,          \
-                                                              splan_threads<SP##L, PP>(), st);
-      CDX_X_PLANS(CDX_CASE)
-#undef CDX_CASE
-      default:
-        break;
-    }
-  if (fx.has_gx) {
+  if (g.pair) {
     bool done = false;
-    const int rc = xgen_update(g, fx, S, Y, Xout, G, dots, w, lam_next, eps, st, &done);
+    const int rc = pxgen_update(pair_geom(g), fx.d_pair, S, Y, Xout, G, dots, &w, lam_next, eps, st,
+                                &done);
     if (done || rc) return rc;
   }
+  if (fx.has_tc && dft_form() == 1)
+    return launch_xtc_update(g, fx.tc, S, Y, Xout, G, dots, w, lam_next, eps, fx.tc.d_err, st);
   const int P = x_pairs(g.nx);
   return x_update_go<GenericRunner>(g, fx.dev, S, Y, Xout, G, dots, w, lam_next, eps, P,
                                     threads_for((long long)P * g.nx), st);

@@ -1,5 +1,6 @@
 // y pass of the 3D transforms: complex FFTs along y of every (kx, z) row.
 #include "decon_common.cuh"
+#include "pair_layout.cuh"
 
 namespace cdx {
 
@@ -52,6 +53,7 @@ static int y_dispatch(const Geom& g, const FftLen& fy, float2* S, cudaStream_t s
 }
 
 int launch_y_pass(const Geom& g, const FftLen& fy, float2* S, bool inverse, cudaStream_t st) {
+  if (g.pair) return launch_py(pair_geom(g), fy, S, inverse, st);
   return inverse ? y_dispatch<true>(g, fy, S, st) : y_dispatch<false>(g, fy, S, st);
 }
 

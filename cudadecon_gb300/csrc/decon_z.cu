@@ -1,6 +1,7 @@
 // z pass: forward FFT along z, OTF multiply (interpolated on the fly),
 // inverse FFT along z.
 #include "decon_common.cuh"
+#include "pair_layout.cuh"
 
 namespace cdx {
 
@@ -215,6 +216,7 @@ static int z_go_static(const Geom& g, const FftDev& f, float2* S, const OtfDev& 
 
 int launch_z_pass(const Geom& g, const FftLen& fz, float2* S, const OtfDev& otf, bool conj,
                   cudaStream_t st, bool fwd_only) {
+  if (g.pair) return launch_pz(pair_geom(g), fz, S, otf, conj, st, fwd_only);
   if (fz.has_static) switch (g.nz) {
 #define CDX_CASE(L, WW)                                                                    \
   case L:                                                                                  \

@@ -13,13 +13,27 @@ namespace cdx {
 // cuFFT's [z][y][kx].  Each plane holds the (z, y) samples of one kx column,
 // so the y pass reads contiguous rows, the z pass reads 128-byte runs, and
 // the x passes write and read transposed 16-byte (two-row) groups.
+// The paired layout (pair_layout.cuh) at height ny: which row shares a complex
+// row with row y (y + pair_split), and the slots per half row.
+__host__ __device__ inline constexpr int pair_split(int ny) {
+  return ny < 4 ? 2 : ny % 4 == 0 ? ny / 2 : ((ny + 1) / 2 + 3) / 4 * 4;
+}
+__host__ __device__ inline constexpr int pair_half(int ny) { return (pair_split(ny) / 2 + 3) / 4 * 4; }
+
 struct Geom {
   int nx, ny, nz;
   int nxh;         // nx/2 + 1
   int nyp;         // ny rounded up to even
   long long plane; // nz * nyp complex elements per kx plane
+  // 1: the spectrum is in the paired layout (pair_layout.cuh) and the paired
+  // passes run; eo: that layout's column order (choose_layout)
+  int pair = 0, eo = 0;
   long long nvox() const { return (long long)nx * ny * nz; }
-  long long spec_elems() const { return (long long)nxh * plane; }
+  // complex elements of a buffer that holds either layout
+  long long spec_elems() const {
+    const int wide = 4 * pair_half(ny);  // 2 hp slots of two complex elements
+    return (long long)nxh * nz * (wide > nyp ? wide : nyp);
+  }
 };
 Geom make_geom(int nx, int ny, int nz);
 
@@ -31,6 +45,7 @@ struct OtfDev {
   const float4* tz;   // mode 0: [nz][nr] OTF resampled along kz, scaled by 1/N, as
                       // pairs (value at ir, value at ir + 1; 0 past the table)
   const float2* full; // mode 1: spectrum-layout OTF, scaled by 1/N
+  const float* h0;    // the raw OTF's value at frequency 0 (real part)
 };
 
 // Raw OTF as read from file, described like the reference's
@@ -59,40 +74,47 @@ void tc_tables_free(TcTables& t);
 int dft_form();
 void set_dft_form(int form);
 
-// FFT plan for one length (host side owns the twiddle table).
-// When the length is in the registry of specialised plans (static_plans.cuh),
-// sdev holds that plan (its radices and twiddle table) as well.
+// Which axis a length is transformed along (its tables differ).
+enum class Axis { x, y, z };
+
+// FFT plan for one length on one axis (host side owns the twiddle tables).
+// dev is the generic engine's plan; when the length is in the registry of
+// specialised y and z plans (static_plans.cuh), sdev holds that plan.
 struct FftLen {
   FftDev dev;
   float2* d_tw = nullptr;
   bool has_static = false;
   FftDev sdev;
   float2* d_tws = nullptr;
-  // the x ratio / x update plan where it differs from the registered one
-  bool has_xr = false;
-  FftDev xrdev;
-  float2* d_twxr = nullptr;
-  // the generated x-pass plan of the length, if it has one
-  bool has_gx = false;
-  FftDev gxdev;
-  float2* d_twgx = nullptr;
   // the generated z-pass plan of the length, if it has one
   bool has_gz = false;
   FftDev gzdev;
   float2* d_twgz = nullptr;
+  // twiddles of the paired plan (fft_pair.cuh), if the length has one; y: the
+  // column order it leaves (PairGeom::eo)
+  float2* d_pair = nullptr;
+  int pair_eo = 0;
   // the tensor-core plan of the length, if it has one
   bool has_tc = false;
   TcTables tc;
 };
-int fft_len_init(FftLen& f, int L);
+int fft_len_init(FftLen& f, int L, Axis axis);
 void fft_len_free(FftLen& f);
 bool fft_len_supported(int L);
+// Set the layout fields of g for the passes of a grid: the paired passes where
+// x has a plan for them, unless the mixed-precision form transforms its rows
+// on the tensor cores (whose x passes use the plain layout).
+void choose_layout(Geom& g, const FftLen& fx, const FftLen& fy);
+
+// Multiprocessors of the current device.
+int sm_count();
 
 // Per-session device state for the Biggs-Andrews loop.
 struct RLWork {
   double* partials = nullptr;   // 2 * max_blocks (16 bytes per x-pass block)
   float* lam = nullptr;         // two slots: lambda used by iteration k is lam[k & 1]
   int max_blocks = 0;
+  const float* h0 = nullptr;    // OTF value at frequency 0 (device)
 };
 
 // ---------------------------------------------------------------- passes

@@ -187,7 +187,7 @@ static int make_otf_device(float* d_psf, int nx, int ny, int nz, const OtfMakePa
   float2 *d_S = nullptr, *d_std = nullptr, *d_ring = nullptr;
   int *d_start = nullptr, *d_offs = nullptr;
   FftLen fx, fy, fz;
-  const Geom g = make_geom(nx, ny, nz);
+  Geom g = make_geom(nx, ny, nz);
   auto cleanup_all = [&]() {
     cudaFree(d_bmax);
     cudaFree(d_bidx);
@@ -278,10 +278,12 @@ static int make_otf_device(float* d_psf, int nx, int ny, int nz, const OtfMakePa
   k_sub<<<grid1(n), 256, 0, st>>>(d_psf, n, background);
   OTF_CHECK(cudaGetLastError());
   // ---- unnormalised 3D R2C (the reference's fftwf_plan_dft_r2c_3d, 135-142)
-  if (fft_len_init(fx, nx) || fft_len_init(fy, ny) || fft_len_init(fz, nz)) {
+  if (fft_len_init(fx, nx, Axis::x) || fft_len_init(fy, ny, Axis::y) ||
+      fft_len_init(fz, nz, Axis::z)) {
     cleanup_all();
     return cudaErrorInvalidValue;
   }
+  choose_layout(g, fx, fy);
   const OtfDev none{};
   OTF_CHECK(cudaMalloc(&d_S, sizeof(float2) * (size_t)g.spec_elems()));
   OTF_CHECK(cudaMalloc(&d_std, sizeof(float2) * (size_t)nxh * ny * nz));

@@ -1,0 +1,88 @@
+// Spectrum layout of the paired passes.
+//
+// Real rows y and y + H (H = ny/2, for ny not divisible by 4 the next multiple
+// of 4, so that the halves start on the same alignment) of a slice are
+// transformed along x as one complex row Z = row[y] + i row[y + H], and two such
+// rows (y = 2m, 2m + 1) form a pair whose lanes a thread transforms together.  The x passes store
+// the packed spectrum Z unsplit; the y pass, which reads both Z[kx] and
+// Z[-kx] of a row, separates the two real rows' spectra as it loads them (the
+// factor 1/2 is folded into the OTF).  For every kx <= nx/2 and z a row of
+// 2 hp float4 slots (hp = H/2 rounded up to 4) holds
+//   between the x and y passes: slot m < hp      Z[kx]  of pair m,
+//                               slot hp + m      Z[-kx] of pair m,
+//   after the forward y pass:   the columns ky of the half spectrum, two per
+//                               slot: (k, k + ny/2) where the y pass splits
+//                               even and odd rows (eo), else (2p, 2p + 1).
+// A slot holds (re lane 0, re lane 1, im lane 0, im lane 1).  Row 0 and, for
+// even nx, row nx/2 are their own mirror image and leave the second half
+// unused.
+//
+// Memory order [z][slot / 4][kx][slot % 4]: the four slots of an x tile's rows
+// are contiguous over all kx (nx/2 + 1 runs of 64 bytes back to back), a y tile
+// of V neighbouring kx reads runs of 64 V bytes, and 16 neighbouring (kx, slot
+// % 4) are a z tile with 256-byte runs.  Stored plane by plane ([kx][z][slot])
+// the x passes read scattered 32- or 64-byte runs: x ratio 82 us with 32-byte
+// and 73 us with 64-byte runs on the 100 x 256 x 756 grid.
+#pragma once
+
+#include "kernels.h"
+
+namespace cdx {
+
+struct PairGeom {
+  int nx, ny, nz, nxh;
+  int H, hp;   // row y shares a complex row with y + H; slots per half row
+  int sb;      // blocks of 4 slots per row: hp / 2
+  int slots;   // column pairs after the y pass
+  int eo;      // 1: columns (k, k + ny/2), 0: (2p, 2p + 1)
+  int zstep;   // slots per z: sb * nxh * 4
+  __host__ __device__ int col(int s, int lane) const { return eo ? s + lane * (ny >> 1) : 2 * s + lane; }
+  // slot s of row (kx, z)
+  __host__ __device__ long long slot(int kx, int z, int s) const {
+    return (long long)z * zstep + ((long long)(s >> 2) * nxh + kx) * 4 + (s & 3);
+  }
+  // float index of the real part of column ky of row (kx, z); the imaginary
+  // part is two floats further
+  __host__ __device__ long long at(int kx, int z, int ky) const {
+    const int h = ny >> 1;
+    const int s = eo ? (ky < h ? ky : ky - h) : ky >> 1;
+    const int lane = eo ? ky >= h : ky & 1;
+    return 4 * slot(kx, z, s) + lane;
+  }
+};
+
+inline PairGeom pair_geom(const Geom& g) {
+  PairGeom p;
+  p.nx = g.nx;
+  p.ny = g.ny;
+  p.nz = g.nz;
+  p.nxh = g.nxh;
+  p.H = pair_split(g.ny);
+  p.hp = pair_half(g.ny);
+  p.sb = p.hp / 2;
+  p.slots = (g.ny + 1) / 2;
+  p.eo = g.eo;
+  p.zstep = p.sb * g.nxh * 4;
+  return p;
+}
+
+#ifdef __CUDACC__
+// Element (kx, z, ky) of a half spectrum in the layout of g.
+__device__ __forceinline__ void st_spec(const Geom& g, const PairGeom& pg, float2* S, int kx, int z,
+                                        int ky, float2 v) {
+  if (g.pair) {
+    float* p = reinterpret_cast<float*>(S) + pg.at(kx, z, ky);
+    p[0] = v.x;
+    p[2] = v.y;
+  } else {
+    S[(long long)kx * g.plane + (long long)z * g.nyp + ky] = v;
+  }
+}
+#endif
+
+// The paired passes (launchers of kernels.h dispatch to them when g.pair).
+int launch_py(const PairGeom& g, const FftLen& fy, float2* S, bool inverse, cudaStream_t st);
+int launch_pz(const PairGeom& g, const FftLen& fz, float2* S, const OtfDev& otf, bool conj,
+              cudaStream_t st, bool fwd_only);
+
+}  // namespace cdx

@@ -4,17 +4,15 @@
 // the lateral cutoff (0 outside) is a convolution, so it runs as the RL
 // convolution passes with this per-frequency factor, built here once per
 // call in the spectrum layout with the 1/N of the inverse transform folded in.
-#include "kernels.h"
+#include "pair_layout.cuh"
 
 namespace cdx {
 
-__global__ void k_wiener_h(Geom g, const float2* __restrict__ otf, int nr, int nzotf, float dkx,
-                           float dky, float kxscale, float kyscale, float kzscale, float rcutoff,
-                           float w, float invN, float2* __restrict__ H) {
-  const int y = blockIdx.x * blockDim.x + threadIdx.x;
-  const int z = blockIdx.y;
-  const int j = blockIdx.z;  // kx
-  if (y >= g.ny) return;
+// The factor at (kx = j, ky of row y, kz of slice z).
+__device__ __forceinline__ float2 wiener_factor(const Geom& g, int j, int y, int z,
+                                                const float2* __restrict__ otf, int nr, int nzotf,
+                                                float dkx, float dky, float kxscale, float kyscale,
+                                                float kzscale, float rcutoff, float w, float invN) {
   const float kz = (float)(z > g.nz / 2 ? z - g.nz : z);
   const float ky = (float)(y > g.ny / 2 ? y - g.ny : y);
   const float kx = (float)j;
@@ -49,16 +47,54 @@ __global__ void k_wiener_h(Geom g, const float2* __restrict__ otf, int nr, int n
     const float s = __fmul_rn(__fdiv_rn(__fsub_rn(1.f, rho), __fadd_rn(amp2, w)), invN);
     h = make_float2(__fmul_rn(o.x, s), __fmul_rn(-o.y, s));  // conj(OTF) * s
   }
-  H[(long long)j * g.plane + (long long)z * g.nyp + y] = h;
+  return h;
+}
+
+__global__ void k_wiener_h(Geom g, const float2* __restrict__ otf, int nr, int nzotf, float dkx,
+                           float dky, float kxscale, float kyscale, float kzscale, float rcutoff,
+                           float w, float invN, float2* __restrict__ H) {
+  const int y = blockIdx.x * blockDim.x + threadIdx.x;
+  const int z = blockIdx.y;
+  const int j = blockIdx.z;  // kx
+  if (y >= g.ny) return;
+  H[(long long)j * g.plane + (long long)z * g.nyp + y] = wiener_factor(
+      g, j, y, z, otf, nr, nzotf, dkx, dky, kxscale, kyscale, kzscale, rcutoff, w, invN);
+}
+
+// The same in the paired layout: a slot (two columns) per thread, consecutive
+// threads on consecutive slots.
+__global__ void k_wiener_h_pair(Geom g, PairGeom pg, const float2* __restrict__ otf, int nr,
+                                int nzotf, float dkx, float dky, float kxscale, float kyscale,
+                                float kzscale, float rcutoff, float w, float invN,
+                                float4* __restrict__ H) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  const int z = blockIdx.y, j = f >> 2, s = blockIdx.z * 4 + (f & 3);
+  if (j >= g.nxh || s >= pg.slots) return;
+  const int y1 = pg.col(s, 1);
+  const float2 a = wiener_factor(g, j, pg.col(s, 0), z, otf, nr, nzotf, dkx, dky, kxscale, kyscale,
+                                 kzscale, rcutoff, w, invN);
+  float2 b = make_float2(0.f, 0.f);
+  if (y1 < g.ny)
+    b = wiener_factor(g, j, y1, z, otf, nr, nzotf, dkx, dky, kxscale, kyscale, kzscale, rcutoff, w,
+                      invN);
+  H[pg.slot(j, z, s)] = make_float4(a.x, b.x, a.y, b.y);
 }
 
 int launch_wiener_h(const Geom& g, const float2* otf, int nr, int nzotf, float dkx, float dky,
                     float kxscale, float kyscale, float kzscale, float rcutoff, float w,
                     float2* H, cudaStream_t st) {
-  const float invN = (float)(1.0 / ((double)g.nx * g.ny * g.nz));
-  dim3 grid(ceil_div(g.ny, 128), g.nz, g.nxh);
-  k_wiener_h<<<grid, 128, 0, st>>>(g, otf, nr, nzotf, dkx, dky, kxscale, kyscale, kzscale,
-                                   rcutoff, w, invN, H);
+  // the paired passes' spectrum is twice the transform
+  const float invN = (float)((g.pair ? 0.5 : 1.0) / ((double)g.nx * g.ny * g.nz));
+  if (g.pair) {
+    const PairGeom pg = pair_geom(g);
+    dim3 grid(ceil_div(4 * g.nxh, 128), g.nz, ceil_div(pg.slots, 4));
+    k_wiener_h_pair<<<grid, 128, 0, st>>>(g, pg, otf, nr, nzotf, dkx, dky, kxscale, kyscale, kzscale,
+                                          rcutoff, w, invN, reinterpret_cast<float4*>(H));
+  } else {
+    dim3 grid(ceil_div(g.ny, 128), g.nz, g.nxh);
+    k_wiener_h<<<grid, 128, 0, st>>>(g, otf, nr, nzotf, dkx, dky, kxscale, kyscale, kzscale, rcutoff,
+                                     w, invN, H);
+  }
   CDX_LAUNCH_CHECK("k_wiener_h");
   return 0;
 }

@@ -3,10 +3,11 @@ the batched workloads' stack sizes that the hand-tuned registry in
 csrc/static_plans.cuh does not already hold: x in [128, 1024], y in
 [128, 512], z in [32, 160].
 
-Writes csrc/static_plans_gen.cuh (the plan lists), csrc/x_gen_dispatch.h
-(the dispatch of the x passes) and csrc/decon_x_gen_<k>.cu (the x-pass
-kernels of the generated x lengths, spread over several units so that the
-build compiles them in parallel).
+Writes csrc/static_plans_gen.cuh (those plan lists), and for the paired passes
+of the plain form (csrc/fft_pair.cuh; x in [128, 2048], y in [32, 1024], z in
+[16, 256]) csrc/pair_plans_gen.cuh (the plans), csrc/x_gen_dispatch.h (their
+dispatch) and csrc/decon_{x,y,z}_gen_<k>.cu (their kernels, spread over several
+units so that the build compiles them in parallel).
 
 Each length has a short list of candidate plans (radix order, pencil batch
 -- rows, row pairs or columns per block -- the register budget behind the
@@ -57,7 +58,9 @@ HERE = Path(__file__).resolve().parent
 OUT = HERE / "csrc" / "static_plans_gen.cuh"
 XDISPATCH = HERE / "csrc" / "x_gen_dispatch.h"
 TUNED = HERE / "tuned_plans.json"
-X_UNITS = 12
+X_UNITS = 20
+Y_UNITS = 8
+Z_UNITS = 8
 N_COLUMNS = 8
 REGX = 16
 PAD_CHOICES = (0, 16, 32, 64, 128)
@@ -312,53 +315,217 @@ def choose(axis: str, L: int, column: int | None,
     return c[0]
 
 
-def x_units(xs: list[int], xplans: dict) -> None:
-    units = [xs[k::X_UNITS] for k in range(X_UNITS)]
+# ---------------------------------------------------------------- paired plans
+PAIR_X_RANGE = (128, 2048)
+PAIR_Y_RANGE = (32, 1024)
+PAIR_Z_RANGE = (16, 256)
+PAIR_MAX_RADIX = 16
+PAIR_Y_RADIX = 16
+PAIR_X_RADIX = 12  # x 256 as 4 8 8 took 17 us in x ratio, as 16 16 30 us
+PAIR_WIDE_RADIX = 27
+PAIRP = HERE / "csrc" / "pair_plans_gen.cuh"
+
+
+def pair_lengths() -> dict[str, list[int]]:
+    def rng(r, points):
+        return [n for n in range(r[0], r[1] + 1) if smooth(n) and pair_radices(*points(n))]
+    return {"x": rng(PAIR_X_RANGE, lambda n: (n, False)), "y": rng(PAIR_Y_RANGE, pair_y_points),
+            "z": rng(PAIR_Z_RANGE, lambda n: (n, False))}
+
+
+def pair_y_points(L: int) -> tuple[int, bool]:
+    """Points of the y transform of height L, and whether it starts even."""
+    return (L // 2, L % 4 == 0) if L % 2 == 0 else (L, False)
+
+
+def pair_radices(L: int, even_first: bool, most: int = PAIR_MAX_RADIX) -> tuple[int, int, int] | None:
+    """Radices (Q0, Q1, Q2) of a paired plan, Q1 = 1 for two.  Two radices of at
+    most `most` points where they exist (one shared round trip less), else the most
+    balanced three; the smallest last (stage C holds the rows' values too), the
+    largest in the middle (stage B touches no global memory).  even_first: Q0
+    is even.  Radices up to 16 and then 27 where that leaves no plan (625 = 5 25 5); None
+    where that does not either (1715 = 5 7^3)."""
+    best = None
+    for a in range(2, PAIR_WIDE_RADIX + 1):
+        if L % a:
+            continue
+        for b in range(1, PAIR_WIDE_RADIX + 1):
+            if (L // a) % b:
+                continue
+            c = L // a // b
+            if not 2 <= c <= PAIR_WIDE_RADIX or (even_first and a % 2):
+                continue
+            two, m = b == 1, max(a, b, c)
+            key = (m > most, m > PAIR_MAX_RADIX, not two, m, 0 if two else -min(a, b, c), c, -b)
+            if best is None or key < best[0]:
+                best = (key, (a, b, c))
+    return best[1] if best else None
+
+
+def _slots(addr: np.ndarray) -> int:
+    """Wavefronts of one 16-byte access per thread: addr (threads,) float4
+    indices, quarter-warps of 8 threads, 8 slots of 16 bytes a wavefront."""
+    a = addr[: len(addr) // 8 * 8].reshape(-1, 8)
+    cnt = np.zeros((len(a), 8), dtype=np.int64)
+    np.add.at(cnt, (np.arange(len(a))[:, None], a % 8), 1)
+    return int(cnt.max(axis=1).sum())
+
+
+@functools.lru_cache(maxsize=None)
+def pair_strides(L: int, rad: tuple[int, int, int], V: int, axis: str, run: int) -> tuple[int, int]:
+    """Strides (S0 of the first digit, VS of a vector) of the shared tile with
+    the fewest modelled wavefronts over the three stages' accesses, smallest
+    first.  x: stage A's threads run over the vectors first.  y: the threads
+    of stages A and C run over `run` butterflies, then the vectors; run = 1
+    (odd heights): vectors slowest, and S0 = Q1 Q2, so that the regrouping
+    passes address elements without a division."""
+    q0, q1, q2 = rad
+    ka, kb, kc = q1 * q2, q0 * q2, q0 * q1
+    best = None
+    for s0 in range(ka, ka + (1 if run == 1 else 8)):
+        for vs in range((q0 - 1) * s0 + ka, (q0 - 1) * s0 + ka + (8 if V > 1 else 1)):
+            if axis == "x":
+                i = np.arange(V * ka)
+                j, v = i // V, i % V
+            else:
+                i = np.arange(V * (ka // run) * run)
+                j, v = (i // (run * V) * run + i % run, i // run % V) if run > 1 else (i % ka, i // ka)
+            cost = q0 * _slots(v * vs + j)
+            if q1 > 1:
+                i = np.arange(V * kb)
+                v, w = i // kb, i % kb
+                cost += q1 * _slots(v * vs + w // q2 * s0 + w % q2)
+            if axis == "x":
+                i = np.arange(V * kc)
+                v, k = i // kc, i % kc
+            else:
+                i = np.arange(V * (kc // run) * run)
+                k, v = (i // (run * V) * run + i % run, i // run % V) if run > 1 else (i % kc, i // kc)
+            cost += q2 * _slots(v * vs + k % q0 * s0 + k // q0 * q2)
+            key = (cost, vs)
+            if best is None or key < best[0]:
+                best = (key, (s0, vs))
+    return best[1]
+
+
+def pair_threads(rad, V: int) -> int:
+    q0, q1, q2 = rad
+    k = max(q1 * q2, q0 * q1, q0 * q2 if q1 > 1 else 0)
+    return (V * k + 31) // 32 * 32
+
+
+def pair_x_warps(L: int, rad, V: int) -> int:
+    """Resident warps per SM of the x passes with V pairs a block: max(4 max(rad)
+    + 24, 8 rad[2] + 12) registers a thread; stage B's twiddles, tile and one copy of the rows in
+    shared memory (227 KB an SM, 1 KB of it kept per block)."""
+    t = pair_threads(rad, V)
+    if t > 1024:
+        return 0
+    smem = 16 * V * (L + 32) + 16 * V * L + 8 * rad[0] * rad[1] + 1024
+    return min(65536 // (t * max(4 * max(rad) + 24, 8 * rad[2] + 12)), 227 * 1024 // smem) * t // 32
+
+
+def pair_z_warps(L: int, rad, V: int) -> int:
+    """Resident warps per SM of the z pass with V column pairs a block: 4
+    max(rad) + 56 registers a thread, twiddles and two tiles in shared memory."""
+    t = pair_threads(rad, V)
+    return min(65536 // (t * (4 * max(rad) + 56)), 227 * 1024 // (8 * L + 32 * V * L + 1024)) * t // 32
+
+
+def pair_plan(axis: str, L: int) -> tuple[int, int, tuple[int, int, int], int, int]:
+    """(transform length, vectors per block, radices, S0, VS) of one length.
+    x: 2 pairs (half a slot block of the layout), 4 where that
+    keeps more warps on an SM (810 at 180 slices of 600 rows: x ratio 308 us
+    with 4, 390 with 2; 1024: 282 and 234); y: neighbouring kx for about 128 threads; z: 16 column pairs
+    (256-byte runs), 8 where that keeps more warps on an SM."""
+    if axis == "x":
+        rad = pair_radices(L, False, PAIR_X_RADIX)
+        V = 4 if pair_x_warps(L, rad, 4) > 1.1 * pair_x_warps(L, rad, 2) else 2
+        return (L, V, rad, *pair_strides(L, rad, V, "x", 0))
+    if axis == "y":
+        n, even = pair_y_points(L)
+        rad = pair_radices(n, even, PAIR_Y_RADIX)
+        V = max(4, round(128 / pair_threads(rad, 8) * 8))
+        return (n, V, rad, *pair_strides(n, rad, V, "y", 4 if n != L else 1))
+    rad = pair_radices(L, False)
+    V = 8 if pair_z_warps(L, rad, 8) > 1.2 * pair_z_warps(L, rad, 16) else 16
+    return (L, V, rad, rad[1] * rad[2], L)
+
+
+def _unit(axis: str, k: int, lens: list[int], body: list[str], header: str) -> None:
+    out = ["// Generated by cudadecon_gb300/gen_plans.py (do not edit): paired "
+           f"{axis}-pass kernels",
+           f"// of the lengths {', '.join(map(str, lens))}.",
+           f'#include "{header}"', '#include "pair_plans_gen.cuh"', '#include "x_gen_dispatch.h"', "",
+           "namespace cdx {", ""] + body + ["}  // namespace cdx", ""]
+    (HERE / "csrc" / f"decon_{axis}_gen_{k}.cu").write_text("\n".join(out))
+
+
+def pair_units() -> dict:
+    """Write the paired plans, their kernels' units and the dispatch."""
+    lens = pair_lengths()
+    plans = {a: {L: pair_plan(a, L) for L in lens[a]} for a in lens}
     kinds = {
-        "fwd": ("const float* X, float* Xm1, const float* lam, int predict, float2* S",
-                "x_fwd_go", "g, fx.gxdev, X, Xm1, lam, predict, S, PP"),
-        "ratio": ("float2* S, const float* raw, float eps",
-                  "x_ratio_go", "g, fx.gxdev, S, raw, eps, PP"),
-        "update": ("const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork& w, "
-                   "float* lam_next, float eps",
-                   "x_update_go", "g, fx.gxdev, S, Y, Xout, G, dots, w, lam_next, eps, PP"),
+        "x": {
+            "pxgen_fwd": ("const PairGeom& g, const float2* tw, const float* X, float* Xm1, "
+                          "const float* lam, int predict, float2* S", "px_fwd_go", X_UNITS),
+            "pxgen_ratio": ("const PairGeom& g, const float2* tw, float2* S, const float* raw, "
+                            "float eps", "px_ratio_go", X_UNITS),
+            "pxgen_update": ("const PairGeom& g, const float2* tw, const float2* S, const float* Y, "
+                             "float* Xout, float* G, int dots, RLWork* w, float* lam_next, "
+                             "float eps", "px_update_go", X_UNITS),
+        },
+        "y": {"pygen": ("const PairGeom& g, const float2* tw, float2* S, bool inv", None, Y_UNITS)},
+        "z": {"pzgen": ("const PairGeom& g, const float2* tw, float2* S, const OtfDev& otf, "
+                        "bool conj", "pz_mode", Z_UNITS)},
     }
+    size = {"x": "g.nx", "y": "g.ny", "z": "g.nz"}
     decl, disp = [], []
-    for kind, (args, go, call) in kinds.items():
-        sig = f"(const Geom& g, const FftLen& fx, {args}, cudaStream_t st, bool* done)"
-        for k in range(X_UNITS):
-            decl.append(f"int xgen_{kind}_{k}{sig};")
-        names = [a.split()[-1].lstrip("*&") for a in args.split(", ")]
-        fwdargs = ", ".join(["g", "fx"] + names + ["st", "done"])
-        body = "\n".join(f"  if ((rc = xgen_{kind}_{k}({fwdargs})) || *done) return rc;"
-                         for k in range(X_UNITS))
-        disp.append(f"inline int xgen_{kind}{sig} {{\n  int rc = 0;\n  *done = false;\n{body}\n"
-                    f"  return 0;\n}}")
+    for axis, ks in kinds.items():
+        tail = "cudaStream_t st, bool fwd_only, bool* done" if axis == "z" else "cudaStream_t st, bool* done"
+        units: dict[int, list[str]] = {}
+        for name, (args, go, n) in ks.items():
+            names = [a.split()[-1].lstrip("*&") for a in (args + ", " + tail).split(", ")]
+            for k in range(n):
+                decl.append(f"int {name}_{k}({args}, {tail});")
+                body = units.setdefault(k, [])
+                body.append(f"int {name}_{k}({args}, {tail}) {{")
+                body.append(f"  switch ({size[axis]}) {{")
+                for L in lens[axis][k::n]:
+                    V = plans[axis][L][1]
+                    fn = go or ("py_eo_go" if L % 2 == 0 else "py_zz_go")
+                    body.append(f"    case {L}:")
+                    body.append("      *done = true;")
+                    body.append(f"      return {fn}<PP{axis.upper()}{L}, {V}>({', '.join(names[:-1])});")
+                body += ["    default:", "      return 0;", "  }", "}", ""]
+            calls = "\n".join(f"  if ((rc = {name}_{k}({', '.join(names)})) || *done) return rc;"
+                              for k in range(n))
+            disp.append(f"inline int {name}({args}, {tail}) {{\n  int rc = 0;\n  *done = false;\n"
+                        f"{calls}\n  return 0;\n}}")
+        hdr = {"x": "decon_px.cuh", "y": "decon_py.cuh", "z": "decon_pz.cuh"}[axis]
+        for k, body in units.items():
+            _unit(axis, k, lens[axis][k::len(units)], body, hdr)
     XDISPATCH.write_text(
         "// Generated by cudadecon_gb300/gen_plans.py (do not edit): dispatch of the\n"
-        "// x passes of the generated x lengths to the units decon_x_gen_<k>.cu.\n"
-        "// Each function sets *done when its length has a generated plan.\n"
-        "#pragma once\n\n#include \"kernels.h\"\n\nnamespace cdx {\n\n" + "\n".join(decl) +
+        "// paired passes to the units decon_{x,y,z}_gen_<k>.cu.  Each function sets\n"
+        "// *done when its length has a plan.\n"
+        "#pragma once\n\n#include \"pair_layout.cuh\"\n\nnamespace cdx {\n\n" + "\n".join(decl) +
         "\n\n" + "\n\n".join(disp) + "\n\n}  // namespace cdx\n")
-    for k, lens in enumerate(units):
-        out = ["// Generated by cudadecon_gb300/gen_plans.py (do not edit): x-pass kernels",
-               f"// of the generated x lengths {', '.join(map(str, lens))}.",
-               '#include "decon_x_kernels.cuh"', '#include "x_gen_dispatch.h"', "",
-               "namespace cdx {", ""]
-        for kind, (args, go, call) in kinds.items():
-            out.append(f"int xgen_{kind}_{k}(const Geom& g, const FftLen& fx, {args}, "
-                       f"cudaStream_t st, bool* done) {{")
-            out.append("  switch (g.nx) {")
-            for L in lens:
-                _, P, rx, (b0, b1) = xplans[L]
-                c = call.replace("PP", str(P))
-                out.append(f"    case {L}:")
-                out.append("      *done = true;")
-                out.append(f"      return {go}<StaticRunner<SPX{L}, {P}, false, false, {rx}, {b0}, "
-                           f"{b1}>>({c}, splan_threads<SPX{L}, {P}>(), st);")
-            out += ["    default:", "      return 0;", "  }", "}", ""]
-        out += ["}  // namespace cdx", ""]
-        (HERE / "csrc" / f"decon_x_gen_{k}.cu").write_text("\n".join(out))
+    out = ["// Generated by cudadecon_gb300/gen_plans.py (do not edit): plans of the paired",
+           "// passes, PP<axis><length> = PPlan<points, Q0, Q1, Q2, S0, VS> (fft_pair.cuh).  A",
+           "// y plan of an even height transforms half of it.",
+           "#pragma once", "", '#include "fft_pair.cuh"', "", "namespace cdx {", ""]
+    for axis in "xyz":
+        for L, (n, V, rad, s0, vs) in plans[axis].items():
+            out.append(f"using PP{axis.upper()}{L} = PPlan<{n}, {rad[0]}, {rad[1]}, {rad[2]}, {s0}, {vs}>;")
+        out += ["", f"// length, points, vectors per block, radices of the {axis} plans",
+                f"#define CDX_P{axis.upper()}_PLANS(F) \\"]
+        out += [f"  F({L}, {n}, {V}, {rad[0]}, {rad[1]}, {rad[2]}) \\"
+                for L, (n, V, rad, s0, vs) in plans[axis].items()]
+        out += [""]
+    out += ["}  // namespace cdx", ""]
+    (HERE / "csrc" / PAIRP.name).write_text("\n".join(out))
+    return plans
 
 
 def generate(column: int | None = None) -> dict:
@@ -385,14 +552,11 @@ def generate(column: int | None = None) -> dict:
                                       for L, c in plans["y"].items()])
     lines += block("CDX_GEN_Z_SPLANS", [f"{L}, {', '.join(map(str, c[0]))}"
                                         for L, c in plans["z"].items()])
-    lines += block("CDX_GEN_X_SPLANS", [f"{L}, {', '.join(map(str, c[0]))}"
-                                        for L, c in plans["x"].items()])
-    lines += block("CDX_GEN_X_PAIRS", [f"{L}, {c[1]}" for L, c in plans["x"].items()])
     lines += block("CDX_GEN_Y_PLANS", [f"{L}, {c[1]}, {c[2]}, {c[3][0]}, {c[3][1]}"
                                        for L, c in plans["y"].items()])
     lines += block("CDX_GEN_Z_PLANS", [f"{L}, {c[1]}, {c[2]}" for L, c in plans["z"].items()])
     OUT.write_text("\n".join(lines) + "\n")
-    x_units(lens["x"], plans["x"])
+    pair_units()
     return plans
 
 
