@@ -11,6 +11,7 @@
 #include "kernels.h"
 
 #include <math.h>
+#include <type_traits>
 
 namespace cdx {
 
@@ -280,40 +281,69 @@ int mean_above_background(const float* img, long long n, double* d_tmp, unsigned
 // the source coordinate in double with one fused multiply-add, rounded once
 // to float; the blend (1-offset)*a + offset*b with the first product fused.
 // The source coordinate depends on (xout, zout) only, so each thread
-// evaluates it once (in double, as the reference does per voxel) and then
-// walks kGeomRows rows of y; GB300's FP64 rate is a small fraction of its
-// FP32 rate.
+// evaluates it once (in double, as the reference does per voxel; GB300's FP64
+// rate is a small fraction of its FP32 rate) and then walks rows of y: 16, or
+// 32 where that still leaves every SM its blocks.  Bound by the bytes it reads
+// and writes: 101x256x512 -> 756 columns takes 30.8 us (131 MB, 4.2 TB/s)
+// against 45.1 us with 16 rows and the loads of one row at a time; 64 rows
+// 32.8 us, 256 rows 37.4 us (too few warps).
 constexpr int kGeomRows = 16;
+constexpr int kDeskewRows = 32;
+constexpr int kDeskewBatch = 16;
 
-__global__ void k_deskew(const float* __restrict__ in, int nx, int ny, int nz,
-                         float* __restrict__ out, int nxOut, int extraShift, double deskewFactor,
-                         float padVal) {
-  const unsigned xout = blockIdx.x * blockDim.x + threadIdx.x;
+// The rows of a thread in batches whose loads are all asked for before the
+// first is used: n rows left, `full` a compile-time true for whole batches.
+template <int B, class F>
+__device__ __forceinline__ void walk_rows(int rows, const F& f) {
+  for (; rows >= B; rows -= B) f(B, std::true_type{});
+  if (rows > 0) f(rows, std::false_type{});
+}
+
+__global__ void __launch_bounds__(128) k_deskew(const float* __restrict__ in, int nx, int ny, int nz,
+                                                float* __restrict__ out, int nxOut, int extraShift,
+                                                double deskewFactor, float padVal, int rows) {
+  const unsigned xout = blockIdx.x * 128 + threadIdx.x;
   const unsigned zout = blockIdx.y;
-  const unsigned y0 = blockIdx.z * kGeomRows;
+  const unsigned y0 = blockIdx.z * rows;
   if (xout >= (unsigned)nxOut) return;
   const double a = __dadd_rn(__dsub_rn((double)xout, nxOut / 2.), (double)extraShift);
   const double b = __dsub_rn((double)zout, nz / 2.);
   const float xin = __double2float_rn(__dadd_rn(__fma_rn(-deskewFactor, b, a), nx / 2.));
-  const unsigned y1 = min(y0 + kGeomRows, (unsigned)ny);
+  const int todo = min(rows, ny - (int)y0);
+  float* dst = out + ((size_t)zout * ny + y0) * nxOut + xout;
   if (xin >= 0 && xin < nx - 1) {
     const float fl = floorf(xin);
     const float offset = __fsub_rn(xin, fl);
     const float w0 = __fsub_rn(1.f, offset);
-    for (unsigned y = y0; y < y1; ++y) {
-      const size_t indin = ((size_t)zout * ny + y) * nx + (unsigned int)fl;
-      out[((size_t)zout * ny + y) * nxOut + xout] =
-          __fmaf_rn(w0, __ldg(in + indin), __fmul_rn(offset, __ldg(in + indin + 1)));
-    }
+    const float* src = in + ((size_t)zout * ny + y0) * nx + (unsigned int)fl;
+    walk_rows<kDeskewBatch>(todo, [&](int n, auto full) {
+      constexpr bool kFull = decltype(full)::value;
+      float a[kDeskewBatch], b[kDeskewBatch];
+#pragma unroll
+      for (int u = 0; u < kDeskewBatch; ++u)
+        if (kFull || u < n) {
+          a[u] = __ldg(src + (size_t)u * nx);
+          b[u] = __ldg(src + (size_t)u * nx + 1);
+        }
+#pragma unroll
+      for (int u = 0; u < kDeskewBatch; ++u)
+        if (kFull || u < n) dst[(size_t)u * nxOut] = __fmaf_rn(w0, a[u], __fmul_rn(offset, b[u]));
+      src += (size_t)kDeskewBatch * nx;
+      dst += (size_t)kDeskewBatch * nxOut;
+    });
   } else {
-    for (unsigned y = y0; y < y1; ++y) out[((size_t)zout * ny + y) * nxOut + xout] = padVal;
+    for (int y = 0; y < todo; ++y) dst[(size_t)y * nxOut] = padVal;
   }
 }
 
 int launch_deskew(const float* in, int nx, int ny, int nz, double deskewFactor, float* out,
                   int nxOut, int extraShift, float padVal, cudaStream_t st) {
-  dim3 grid(ceil_div(nxOut, 128), nz, ceil_div(ny, kGeomRows));
-  k_deskew<<<grid, 128, 0, st>>>(in, nx, ny, nz, out, nxOut, extraShift, deskewFactor, padVal);
+  int rows = kGeomRows;
+  while (rows < kDeskewRows && (long long)ceil_div(nxOut, 128) * nz * ceil_div(ny, 2 * rows) >= 2048)
+    rows *= 2;
+  const dim3 grid(ceil_div(nxOut, 128), nz, ceil_div(ny, rows));
+  k_deskew<<<grid, 128, 0, st>>>(in, nx, ny, nz, out, nxOut, extraShift, deskewFactor, padVal,
+                                 rows);
   CDX_LAUNCH_CHECK("k_deskew");
   return 0;
 }
@@ -326,22 +356,35 @@ struct Rot4 {
   float p[4];
 };
 
-// Arithmetic written out as the reference's nvcc build evaluates it (pinned
-// against the reference kernel on the GPU): each coordinate is
-// fmaf(r0, zc, r1*xc) in float, then the half size is added in double and
-// the sum rounded to float; each of the three blends fuses its first product.
-__global__ void k_rotate(const float* __restrict__ in, int nx_in, int ny, int nz_in,
+// Arithmetic as the reference's nvcc build evaluates it (pinned against the
+// reference kernel on the GPU): each coordinate is fmaf(r0, zc, r1*xc) in
+// float, then the half size is added in double and the sum rounded to float;
+// each of the three blends fuses its first product.  The additions are in
+// float here and give the same numbers: half sizes and centred indices are
+// exact in float, and a sum of two floats rounded to double and then to float
+// is the float sum, since 53 >= 2 * 24 + 2 (Figueroa, "When is double rounding
+// innocuous?", 1995).
+// A warp takes kRotX columns of kRotZ output slices: at the usual 30 degrees
+// 32 columns of one slice fall on 16 or more input slices, each a cache line
+// of its own, 16 columns of two on half as many.  The four loads of a voxel
+// through L1 bound it: 101x256x756 -> 152x256x724 takes 43.7 us, 50.5 us at
+// 32 x 1 columns, 47.0 at 8 x 4, 74.2 at 4 x 8, and 73.7 us before, with the
+// coordinates in double and the loads of one row at a time.
+constexpr int kRotX = 16, kRotZ = 32 / kRotX, kRotWarps = 4, kRotBatch = 8;
+
+__global__ void __launch_bounds__(32 * kRotWarps) k_rotate(const float* __restrict__ in, int nx_in, int ny, int nz_in,
                          float* __restrict__ out, int nx_out, int nz_out, Rot4 rot) {
-  const unsigned xout = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned zout = blockIdx.y;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned xout = (blockIdx.x * kRotWarps + warp) * kRotX + lane % kRotX;
+  const unsigned zout = blockIdx.y * kRotZ + lane / kRotX;
   const unsigned y0 = blockIdx.z * kGeomRows;
-  if (xout >= (unsigned)nx_out) return;
-  const float xc = __double2float_rn(__dsub_rn((double)xout, nx_out / 2.));
-  const float zc = __double2float_rn(__dsub_rn((double)zout, nz_out / 2.));
-  const float zin = __double2float_rn(
-      __dadd_rn((double)__fmaf_rn(rot.p[0], zc, __fmul_rn(rot.p[1], xc)), nz_in / 2.));
-  const float xin = __double2float_rn(
-      __dadd_rn((double)__fmaf_rn(rot.p[2], zc, __fmul_rn(rot.p[3], xc)), nx_in / 2.));
+  if (xout >= (unsigned)nx_out || zout >= (unsigned)nz_out) return;
+  const float xc = __fsub_rn((float)xout, 0.5f * (float)nx_out);
+  const float zc = __fsub_rn((float)zout, 0.5f * (float)nz_out);
+  const float zin =
+      __fadd_rn(__fmaf_rn(rot.p[0], zc, __fmul_rn(rot.p[1], xc)), 0.5f * (float)nz_in);
+  const float xin =
+      __fadd_rn(__fmaf_rn(rot.p[2], zc, __fmul_rn(rot.p[3], xc)), 0.5f * (float)nx_in);
   const size_t nxy_in = (size_t)nx_in * ny;
   const size_t nxy_out = (size_t)nx_out * ny;
   const size_t obase = (size_t)(nz_out - 1 - zout) * nxy_out + xout;
@@ -351,13 +394,31 @@ __global__ void k_rotate(const float* __restrict__ in, int nx_in, int ny, int nz
     const size_t ibase = (size_t)(unsigned)fz * nxy_in + (unsigned)fx;
     const float xo = __fsub_rn(xin, fx), zo = __fsub_rn(zin, fz);
     const float wx = __fsub_rn(1.f, xo), wz = __fsub_rn(1.f, zo);
-    for (unsigned y = y0; y < y1; ++y) {
-      const size_t i00 = ibase + (size_t)y * nx_in;
-      const size_t i10 = i00 + nxy_in;
-      const float a = __fmaf_rn(wx, __ldg(in + i00), __fmul_rn(xo, __ldg(in + i00 + 1)));
-      const float b = __fmaf_rn(wx, __ldg(in + i10), __fmul_rn(xo, __ldg(in + i10 + 1)));
-      out[obase + (size_t)y * nx_out] = __fmaf_rn(wz, a, __fmul_rn(zo, b));
-    }
+    const float* s0 = in + ibase + (size_t)y0 * nx_in;
+    const float* s1 = s0 + nxy_in;
+    float* dst = out + obase + (size_t)y0 * nx_out;
+    walk_rows<kRotBatch>(y1 - y0, [&](int n, auto full) {
+      constexpr bool kFull = decltype(full)::value;
+      float v[kRotBatch][4];
+#pragma unroll
+      for (int u = 0; u < kRotBatch; ++u)
+        if (kFull || u < n) {
+          v[u][0] = __ldg(s0 + (size_t)u * nx_in);
+          v[u][1] = __ldg(s0 + (size_t)u * nx_in + 1);
+          v[u][2] = __ldg(s1 + (size_t)u * nx_in);
+          v[u][3] = __ldg(s1 + (size_t)u * nx_in + 1);
+        }
+#pragma unroll
+      for (int u = 0; u < kRotBatch; ++u)
+        if (kFull || u < n) {
+          const float a = __fmaf_rn(wx, v[u][0], __fmul_rn(xo, v[u][1]));
+          const float b = __fmaf_rn(wx, v[u][2], __fmul_rn(xo, v[u][3]));
+          dst[(size_t)u * nx_out] = __fmaf_rn(wz, a, __fmul_rn(zo, b));
+        }
+      s0 += (size_t)kRotBatch * nx_in;
+      s1 += (size_t)kRotBatch * nx_in;
+      dst += (size_t)kRotBatch * nx_out;
+    });
   } else {
     for (unsigned y = y0; y < y1; ++y) out[obase + (size_t)y * nx_out] = 0.f;
   }
@@ -367,8 +428,9 @@ int launch_rotate(const float* in, int nx_in, int ny, int nz_in, const float* ro
                   int nx_out, int nz_out, cudaStream_t st) {
   Rot4 r;
   for (int i = 0; i < 4; ++i) r.p[i] = rot_host[i];
-  dim3 grid(ceil_div(nx_out, 128), nz_out, ceil_div(ny, kGeomRows));
-  k_rotate<<<grid, 128, 0, st>>>(in, nx_in, ny, nz_in, out, nx_out, nz_out, r);
+  const dim3 grid(ceil_div(nx_out, kRotX * kRotWarps), ceil_div(nz_out, kRotZ),
+                  ceil_div(ny, kGeomRows));
+  k_rotate<<<grid, 32 * kRotWarps, 0, st>>>(in, nx_in, ny, nz_in, out, nx_out, nz_out, r);
   CDX_LAUNCH_CHECK("k_rotate");
   return 0;
 }

@@ -82,30 +82,61 @@ int launch_stitch(const float* tile, float* out, unsigned char* weight, int nx, 
 
 // MaxIntProj (linearDecon.cpp:1434-1473): maximum along axis 0 (x), 1 (y) or
 // 2 (z), starting from -1e10; outputs (ny, nz), (nx, nz), (nx, ny) images,
-// first size fastest.
-__global__ void k_mip(const float* __restrict__ in, int nx, int ny, int nz, int axis,
-                      float* __restrict__ out) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;  // fastest output index
-  const int b = blockIdx.y;
+// first size fastest.  NaN is never taken (fmaxf returns the other operand, as
+// the comparison p > m does).
+constexpr int kMipBatch = 8;  // loads in flight per thread
+constexpr int kMipCols = 128, kMipSplit = 8;  // axes 1 and 2: columns of a block, its rows at most
+
+// Axis 0: a warp per row, so that its loads are contiguous.  152x256x724: 19 us
+// for the call (112 MB, L2-resident in part) against 50 us with a thread per row.
+__global__ void __launch_bounds__(256) k_mip_x(const float* __restrict__ in, int nx,
+                                               long long rows, float* __restrict__ out) {
+  const long long r = blockIdx.x * 8LL + (threadIdx.x >> 5);
+  if (r >= rows) return;
+  const float* p = in + r * nx;
   float m = -1e10f;
-  if (axis == 0) {
-    if (a >= ny) return;
-    const float* p = in + ((long long)b * ny + a) * nx;
-    for (int x = 0; x < nx; ++x)
-      if (p[x] > m) m = p[x];
-    out[(long long)b * ny + a] = m;
-  } else if (axis == 1) {
-    if (a >= nx) return;
-    const float* p = in + (long long)b * ny * nx + a;
-    for (int y = 0; y < ny; ++y)
-      if (p[(long long)y * nx] > m) m = p[(long long)y * nx];
-    out[(long long)b * nx + a] = m;
-  } else {
-    if (a >= nx) return;
-    const float* p = in + (long long)b * nx + a;
-    for (int z = 0; z < nz; ++z)
-      if (p[(long long)z * ny * nx] > m) m = p[(long long)z * ny * nx];
-    out[(long long)b * nx + a] = m;
+  for (int x0 = threadIdx.x & 31; x0 < nx; x0 += 32 * kMipBatch) {
+    float v[kMipBatch];
+#pragma unroll
+    for (int u = 0; u < kMipBatch; ++u) v[u] = x0 + 32 * u < nx ? __ldg(p + x0 + 32 * u) : -1e10f;
+#pragma unroll
+    for (int u = 0; u < kMipBatch; ++u) m = fmaxf(m, v[u]);
+  }
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) out[r] = m;
+}
+
+// Axes 1 and 2: the maximum of n values `step` apart for kMipCols neighbouring x and
+// one `slow` index (z or y, `slow_step` apart); blockDim.y threads share a column: as
+// many as keep all of the grid resident, so that it walks the planes together.
+// 152x256x724: 21.9 and 22.6 us (25.4 and 20.1 us with one thread a column and
+// no batches; 24.6 us on axis 2 where the grid takes two waves).
+__global__ void __launch_bounds__(kMipCols* kMipSplit)
+k_mip_col(const float* __restrict__ in, int nx, int n, long long step, long long slow_step,
+          float* __restrict__ out) {
+  __shared__ float red[kMipSplit][kMipCols];
+  const unsigned cols = (nx + kMipCols - 1) / kMipCols, slow = blockIdx.x / cols;
+  const int x = (blockIdx.x - slow * cols) * kMipCols + threadIdx.x;
+  const int part = threadIdx.y, split = blockDim.y;
+  float m = -1e10f;
+  if (x < nx) {
+    const float* p = in + slow * slow_step + x;
+    for (int i0 = part; i0 < n; i0 += split * kMipBatch) {
+      float v[kMipBatch];
+#pragma unroll
+      for (int u = 0; u < kMipBatch; ++u) {
+        const int i = i0 + u * split;
+        v[u] = i < n ? __ldg(p + i * step) : -1e10f;
+      }
+#pragma unroll
+      for (int u = 0; u < kMipBatch; ++u) m = fmaxf(m, v[u]);
+    }
+  }
+  red[part][threadIdx.x] = m;
+  __syncthreads();
+  if (part == 0 && x < nx) {
+    for (int i = 1; i < split; ++i) m = fmaxf(m, red[i][threadIdx.x]);
+    out[(long long)slow * nx + x] = m;
   }
 }
 
@@ -114,10 +145,17 @@ int launch_mip(const float* in, int nx, int ny, int nz, int axis, float* out, cu
     set_error("mip", "axis must be 0, 1 or 2");
     return cudaErrorInvalidValue;
   }
-  const int fast = axis == 0 ? ny : nx;
-  const int slow = axis == 2 ? ny : nz;
-  dim3 grid(ceil_div(fast, 128), slow);
-  k_mip<<<grid, 128, 0, st>>>(in, nx, ny, nz, axis, out);
+  if (axis == 0) {
+    const long long rows = (long long)ny * nz;
+    k_mip_x<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(in, nx, rows, out);
+  } else {
+    const long long plane = (long long)ny * nx;
+    const int n = axis == 1 ? ny : nz, slow = axis == 1 ? nz : ny;
+    int split = 1;
+    while (split < kMipSplit && (long long)nx * slow * 2 * split <= 2048LL * sm_count()) split *= 2;
+    k_mip_col<<<ceil_div(nx, kMipCols) * slow, dim3(kMipCols, split), 0, st>>>(
+        in, nx, n, axis == 1 ? nx : plane, axis == 1 ? plane : nx, out);
+  }
   CDX_LAUNCH_CHECK("k_mip");
   return 0;
 }
