@@ -124,13 +124,21 @@ struct Session {
   // work buffers
   GridPlan plan;
   DevBuf<unsigned short> u16in;
-  DevBuf<float> pre, Xa, Xb, G, raw, rotbuf, res_stage, desk_stage, conv_tmp;
+  DevBuf<float> pre, Xa, Xb, G, raw, rotbuf, res_stage, desk_stage;
   // Y tiling (cdx_RL_tiled): the whole raw stack, one tile, the stitched
   // output and its blend weights
   DevBuf<unsigned short> tile_raw, tile_in;
   DevBuf<float> tile_out;
   DevBuf<unsigned char> tile_weight;
   DevBuf<float2> S;
+  // Wiener filter: spectrum, filter factors, background-subtracted volume
+  DevBuf<float2> wiener_S, wiener_H;
+  DevBuf<float> wiener_in;
+  void release_wiener() {
+    wiener_S.release();
+    wiener_H.release();
+    wiener_in.release();
+  }
   DevBuf<double> partials, stat_d;
   DevBuf<unsigned> stat_u;
   DevBuf<float> lam;
@@ -219,7 +227,7 @@ static void release_all(Session& s) {
   s.rotbuf.release();
   s.res_stage.release();
   s.desk_stage.release();
-  s.conv_tmp.release();
+  s.release_wiener();
   s.tile_raw.release();
   s.tile_in.release();
   s.tile_out.release();
@@ -1374,7 +1382,7 @@ void RL_cleanup(void) {
   s.rotbuf.release();
   s.desk_stage.release();
   s.res_stage.release();
-  s.conv_tmp.release();
+  s.release_wiener();
   s.tile_raw.release();
   s.tile_in.release();
   s.tile_out.release();
@@ -1711,25 +1719,30 @@ int cdx_wiener_device(const float* in, float* out, int nx, int ny, int nz, float
   const float rcutoff = 2 * NA / wavelength;
   const float w = wiener * wiener;
   const float kxscale = dkx / s.dkx_otf, kyscale = dky / s.dkx_otf, kzscale = dkz / s.dkz_otf;
-  DevBuf<float2> S, H;
-  DevBuf<float> tmp;
+  // The workspaces stay with the session up to kWienerKeep bytes, until
+  // RL_cleanup: at 100x256x756 the passes take 280 us, and allocating and
+  // freeing the three around them took another 440 us.  Every call ends
+  // synchronised, so calls on different streams can share them.
+  constexpr size_t kWienerKeep = 4ull << 30;
+  const size_t ns = (size_t)g.spec_elems(), nv = (size_t)g.nvox();
   OtfDev hd{};
-  int ok = !(S.ensure((size_t)g.spec_elems()) || H.ensure((size_t)g.spec_elems()) ||
-             tmp.ensure((size_t)g.nvox()));
+  int ok = !(s.wiener_S.ensure(ns) || s.wiener_H.ensure(ns) || s.wiener_in.ensure(nv));
   if (ok) {
+    float2 *S = s.wiener_S.p, *H = s.wiener_H.p;
     hd.mode = 1;
-    hd.full = H.p;
-    ok = !(launch_minus(in, tmp.p, g.nvox(), background, st) ||
+    hd.full = H;
+    ok = !(launch_minus(in, s.wiener_in.p, g.nvox(), background, st) ||
            launch_wiener_h(g, s.raw_otf.p, (int)s.od.nx_otf, (int)s.od.nz_otf, dkx, dky, kxscale,
-                           kyscale, kzscale, rcutoff, w, H.p, st) ||
-           launch_x_fwd(g, p.fx, tmp.p, nullptr, nullptr, 0, S.p, st) ||
-           launch_y_pass(g, p.fy, S.p, false, st) || launch_z_pass(g, p.fz, S.p, hd, false, st) ||
-           launch_y_pass(g, p.fy, S.p, true, st) || launch_x_inv_plain(g, p.fx, S.p, out, st) ||
-           cudaStreamSynchronize(st));
+                           kyscale, kzscale, rcutoff, w, H, st) ||
+           launch_x_fwd(g, p.fx, s.wiener_in.p, nullptr, nullptr, 0, S, st) ||
+           launch_y_pass(g, p.fy, S, false, st) || launch_z_pass(g, p.fz, S, hd, false, st) ||
+           launch_y_pass(g, p.fy, S, true, st) || launch_x_inv_plain(g, p.fx, S, out, st));
+    // also after a failure: earlier passes may still be using the workspaces
+    ok = cudaStreamSynchronize(st) == cudaSuccess && ok;
   }
-  S.release();
-  H.release();
-  tmp.release();
+  const size_t held =
+      sizeof(float2) * (s.wiener_S.n + s.wiener_H.n) + sizeof(float) * s.wiener_in.n;
+  if (!ok || held > kWienerKeep) s.release_wiener();
   return ok;
 }
 

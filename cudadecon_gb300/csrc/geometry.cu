@@ -299,9 +299,9 @@ __device__ __forceinline__ void walk_rows(int rows, const F& f) {
   if (rows > 0) f(rows, std::false_type{});
 }
 
-__global__ void __launch_bounds__(128) k_deskew(const float* __restrict__ in, int nx, int ny, int nz,
-                                                float* __restrict__ out, int nxOut, int extraShift,
-                                                double deskewFactor, float padVal, int rows) {
+__global__ void __launch_bounds__(128)
+k_deskew(const float* __restrict__ in, int nx, int ny, int nz, float* __restrict__ out, int nxOut,
+         int extraShift, double deskewFactor, float padVal, int rows) {
   const unsigned xout = blockIdx.x * 128 + threadIdx.x;
   const unsigned zout = blockIdx.y;
   const unsigned y0 = blockIdx.z * rows;
@@ -339,8 +339,8 @@ __global__ void __launch_bounds__(128) k_deskew(const float* __restrict__ in, in
 int launch_deskew(const float* in, int nx, int ny, int nz, double deskewFactor, float* out,
                   int nxOut, int extraShift, float padVal, cudaStream_t st) {
   int rows = kGeomRows;
-  while (rows < kDeskewRows && (long long)ceil_div(nxOut, 128) * nz * ceil_div(ny, 2 * rows) >= 2048)
-    rows *= 2;
+  const long long columns = (long long)ceil_div(nxOut, 128) * nz;
+  while (rows < kDeskewRows && columns * ceil_div(ny, 2 * rows) >= 2048) rows *= 2;
   const dim3 grid(ceil_div(nxOut, 128), nz, ceil_div(ny, rows));
   k_deskew<<<grid, 128, 0, st>>>(in, nx, ny, nz, out, nxOut, extraShift, deskewFactor, padVal,
                                  rows);
@@ -372,8 +372,9 @@ struct Rot4 {
 // coordinates in double and the loads of one row at a time.
 constexpr int kRotX = 16, kRotZ = 32 / kRotX, kRotWarps = 4, kRotBatch = 8;
 
-__global__ void __launch_bounds__(32 * kRotWarps) k_rotate(const float* __restrict__ in, int nx_in, int ny, int nz_in,
-                         float* __restrict__ out, int nx_out, int nz_out, Rot4 rot) {
+__global__ void __launch_bounds__(32 * kRotWarps)
+k_rotate(const float* __restrict__ in, int nx_in, int ny, int nz_in, float* __restrict__ out,
+         int nx_out, int nz_out, Rot4 rot) {
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned xout = (blockIdx.x * kRotWarps + warp) * kRotX + lane % kRotX;
   const unsigned zout = blockIdx.y * kRotZ + lane / kRotX;
