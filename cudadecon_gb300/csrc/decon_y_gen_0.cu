@@ -43,7 +43,7 @@ int pygen_0(const PairGeom& g, const float2* tw, float2* S, bool inv, cudaStream
       return py_eo_go<PPY490, 4>(g, tw, S, inv, st);
     case 576:
       *done = true;
-      return py_eo_go<PPY576, 4>(g, tw, S, inv, st);
+      return py_eo_go<PPY576, 6>(g, tw, S, inv, st);
     case 675:
       *done = true;
       return py_zz_go<PPY675, 4>(g, tw, S, inv, st);

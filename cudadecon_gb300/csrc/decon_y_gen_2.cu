@@ -37,10 +37,10 @@ int pygen_2(const PairGeom& g, const float2* tw, float2* S, bool inv, cudaStream
       return py_eo_go<PPY360, 8>(g, tw, S, inv, st);
     case 432:
       *done = true;
-      return py_eo_go<PPY432, 4>(g, tw, S, inv, st);
+      return py_eo_go<PPY432, 6>(g, tw, S, inv, st);
     case 504:
       *done = true;
-      return py_eo_go<PPY504, 4>(g, tw, S, inv, st);
+      return py_eo_go<PPY504, 6>(g, tw, S, inv, st);
     case 600:
       *done = true;
       return py_eo_go<PPY600, 4>(g, tw, S, inv, st);

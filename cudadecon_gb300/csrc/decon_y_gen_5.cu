@@ -40,7 +40,7 @@ int pygen_5(const PairGeom& g, const float2* tw, float2* S, bool inv, cudaStream
       return py_eo_go<PPY450, 8>(g, tw, S, inv, st);
     case 540:
       *done = true;
-      return py_eo_go<PPY540, 4>(g, tw, S, inv, st);
+      return py_eo_go<PPY540, 6>(g, tw, S, inv, st);
     case 640:
       *done = true;
       return py_eo_go<PPY640, 4>(g, tw, S, inv, st);

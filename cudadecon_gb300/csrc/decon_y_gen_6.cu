@@ -31,7 +31,7 @@ int pygen_6(const PairGeom& g, const float2* tw, float2* S, bool inv, cudaStream
       return py_eo_go<PPY256, 8>(g, tw, S, inv, st);
     case 324:
       *done = true;
-      return py_eo_go<PPY324, 4>(g, tw, S, inv, st);
+      return py_eo_go<PPY324, 6>(g, tw, S, inv, st);
     case 392:
       *done = true;
       return py_eo_go<PPY392, 8>(g, tw, S, inv, st);
@@ -43,7 +43,7 @@ int pygen_6(const PairGeom& g, const float2* tw, float2* S, bool inv, cudaStream
       return py_eo_go<PPY560, 4>(g, tw, S, inv, st);
     case 648:
       *done = true;
-      return py_eo_go<PPY648, 4>(g, tw, S, inv, st);
+      return py_eo_go<PPY648, 6>(g, tw, S, inv, st);
     case 750:
       *done = true;
       return py_eo_go<PPY750, 4>(g, tw, S, inv, st);

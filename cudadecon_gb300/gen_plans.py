@@ -320,7 +320,7 @@ PAIR_X_RANGE = (128, 2048)
 PAIR_Y_RANGE = (32, 1024)
 PAIR_Z_RANGE = (16, 256)
 PAIR_MAX_RADIX = 16
-PAIR_Y_RADIX = 16
+PAIR_Y_RADIX = 18  # y 324 as 18 9 took 30-37 us a pass on 108 x 324 x 525, as 6 9 3 35-44 us
 PAIR_X_RADIX = 12  # x 256 as 4 8 8 took 17 us in x ratio, as 16 16 30 us
 PAIR_WIDE_RADIX = 27
 PAIRP = HERE / "csrc" / "pair_plans_gen.cuh"
@@ -343,7 +343,7 @@ def pair_radices(L: int, even_first: bool, most: int = PAIR_MAX_RADIX) -> tuple[
     most `most` points where they exist (one shared round trip less), else the most
     balanced three; the smallest last (stage C holds the rows' values too), the
     largest in the middle (stage B touches no global memory).  even_first: Q0
-    is even.  Radices up to 16 and then 27 where that leaves no plan (625 = 5 25 5); None
+    is even.  Radices up to `most` or 16 and then 27 where that leaves no plan (625 = 5 25 5); None
     where that does not either (1715 = 5 7^3)."""
     best = None
     for a in range(2, PAIR_WIDE_RADIX + 1):
@@ -356,7 +356,7 @@ def pair_radices(L: int, even_first: bool, most: int = PAIR_MAX_RADIX) -> tuple[
             if not 2 <= c <= PAIR_WIDE_RADIX or (even_first and a % 2):
                 continue
             two, m = b == 1, max(a, b, c)
-            key = (m > most, m > PAIR_MAX_RADIX, not two, m, 0 if two else -min(a, b, c), c, -b)
+            key = (m > most, m > max(most, PAIR_MAX_RADIX), not two, m, 0 if two else -min(a, b, c), c, -b)
             if best is None or key < best[0]:
                 best = (key, (a, b, c))
     return best[1] if best else None
