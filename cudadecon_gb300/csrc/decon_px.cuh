@@ -164,7 +164,16 @@ struct PX {
   }
   static constexpr int kBlocksFwd = resident_blocks(by_regs(24 + 4 * PL::qmax()), smem_fwd(2));
   static constexpr int kRegsUpd = 24 + 4 * PL::qmax() > 64 ? 24 + 4 * PL::qmax() : 64;
-  static constexpr int kBlocksUpd = resident_blocks(by_regs(kRegsUpd), smem(0));
+  // Row arrays (Y, then G) that the update pass of a large volume has in shared
+  // memory: as many as leave 512 threads an SM, or all that fit beside the
+  // blocks there are without them.  One block of two lost 27% of the pass at 800
+  // columns, two of four (448 threads) 9% at 756, three of eight (192) 13% at
+  // 625; three of four (672) gained 6% at 700, four of eight (512) 3% at 512.
+  static constexpr int blocks_upd(int R) { return resident_blocks(by_regs(kRegsUpd), smem(R)); }
+  static constexpr bool stages(int R) {
+    return blocks_upd(R) * T >= 512 || blocks_upd(R) == blocks_upd(0);
+  }
+  static constexpr int kStaged = stages(2) ? 2 : (stages(1) ? 1 : 0);
   __device__ __forceinline__ static float* rows_fwd(float2* sm, int i) {
     return reinterpret_cast<float*>(tile(sm)) + i * kRows;
   }
@@ -204,9 +213,9 @@ __device__ __forceinline__ void rows_to_spec(const PairGeom& g, C2* x, float4* s
 }
 
 // Packed spectrum -> stages A and B inverse; the tile then holds stage C's
-// inputs.  Waits for the thread's async copies (twiddles, rows) before its
-// first barrier; then() runs before its last.
-template <class PL, int NQ, bool LAST, class Then>
+// inputs.  Waits for the thread's async copies (twiddles, rows), all but
+// the last KEEP groups, before its first barrier; then() runs before its last.
+template <class PL, int NQ, bool LAST, int KEEP = 0, class Then>
 __device__ __forceinline__ void spec_to_tile(const PairGeom& g, float4* sm, const float2* stw,
                                              float4* S, int z, int m0, const Then& then) {
   const int idx = threadIdx.x;
@@ -229,7 +238,7 @@ __device__ __forceinline__ void spec_to_tile(const PairGeom& g, float4* sm, cons
 #pragma unroll
     for (int r = 0; r < PL::Q0; ++r) stp(p + r * PL::S0, y[r]);
   }
-  cp_async_wait_all();
+  cp_async_wait<KEEP>();
   if constexpr (PL::Q1 == 1) then();
   __syncthreads();
   stage_b<PL, NQ, true, false>(sm, stw, then);
@@ -407,8 +416,8 @@ __device__ __forceinline__ void acc_add2(float2& hi, float2& lo, float2 p) {
 
 // Y == nullptr: the plain inverse transform, written to Xout; otherwise h0 is
 // the OTF at frequency 0 (see k_px_ratio).
-template <class PL, int NQ>
-__global__ void __launch_bounds__(PX<PL, NQ>::T, PX<PL, NQ>::kBlocksUpd)
+template <class PL, int NQ, int STAGED>
+__global__ void __launch_bounds__(PX<PL, NQ>::T, PX<PL, NQ>::blocks_upd(STAGED))
 k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y, float* Xout,
             float* G, int dots, float4* partials, const float* h0) {
   using P = PX<PL, NQ>;
@@ -422,17 +431,25 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
   const RowRuns<NQ> runs(g, z, m0);
   const bool vec = Y && runs.vec(Xout) && runs.vec(Y) && runs.vec(G);
   // Y and G were written by kernels that completed before the previous pass
-  // passed its own wait: ask for them in L2 now
+  // passed its own wait: ask for them now, in shared memory (the first STAGED of
+  // them) or in L2 (16-byte walk only: the prefetch takes whole 16-byte units)
+  if constexpr (STAGED > 0) {
+    prefetch_rows<NQ>(g, P::rows(smem, 0), Y, z, m0);
+    if (STAGED > 1 && dots) prefetch_rows<NQ>(g, P::rows(smem, 1), G, z, m0);
+    cp_async_commit();
+  }
   if (vec && threadIdx.x == 0) {
-    l2_prefetch(Y + runs.o, 4 * runs.n0);
-    l2_prefetch(Y + runs.o + runs.h, 4 * runs.n1);
-    if (dots) {
+    if (STAGED < 1) {
+      l2_prefetch(Y + runs.o, 4 * runs.n0);
+      l2_prefetch(Y + runs.o + runs.h, 4 * runs.n1);
+    }
+    if (STAGED < 2 && dots) {
       l2_prefetch(G + runs.o, 4 * runs.n0);
       l2_prefetch(G + runs.o + runs.h, 4 * runs.n1);
     }
   }
   grid_dep_wait();
-  spec_to_tile<PL, NQ, true>(g, sm, stw, S, z, m0, [] {});
+  spec_to_tile<PL, NQ, true, STAGED ? 1 : 0>(g, sm, stw, S, z, m0, [] {});
   // stage C, its samples as rows over the tile (all of it read by then)
   const int idx = threadIdx.x;
   const int q = idx / PL::KC, k = idx - q * PL::KC;
@@ -453,6 +470,7 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
       for (int r = 0; r < PL::Q2; ++r) sts_rows<NQ, PL::L>(rows, q, k + r * PL::KC, x[r]);
     }
   }
+  if constexpr (STAGED > 0) cp_async_wait_all();
   __syncthreads();
   grid_dep_launch_small();
   // Estimate update (currEstimate_kernel + currPrevDiff_kernel,
@@ -492,8 +510,12 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
         const int i = i0 + u * P::T;
         at[u] = (i < n0 ? o0 : o1) + i;
         if (i < n) {
-          y[u] = __ldcs(reinterpret_cast<const float4*>(Y) + at[u]);
-          if (dots) go[u] = __ldcs(reinterpret_cast<const float4*>(G) + at[u]);
+          const int f = i < n0 ? i : i - n0 + NQ * PL::L / 2;
+          y[u] = STAGED > 0 ? reinterpret_cast<const float4*>(P::rows(smem, 0))[f]
+                            : __ldcs(reinterpret_cast<const float4*>(Y) + at[u]);
+          if (dots)
+            go[u] = STAGED > 1 ? reinterpret_cast<const float4*>(P::rows(smem, 1))[f]
+                               : __ldcs(reinterpret_cast<const float4*>(G) + at[u]);
         }
       }
 #pragma unroll
@@ -521,8 +543,9 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
         float v = 0.f, w = 0.f;
         if (i < total) {
           const long long at = (i < runs.n0 ? runs.o : o1) + i;
-          v = __ldcs(Y + at);
-          if (dots) w = __ldcs(G + at);
+          const int f = i < runs.n0 ? i : i - runs.n0 + 2 * NQ * PL::L;
+          v = STAGED > 0 ? P::rows(smem, 0)[f] : __ldcs(Y + at);
+          if (dots) w = STAGED > 1 ? P::rows(smem, 1)[f] : __ldcs(G + at);
         }
         (u & 1 ? y[u / 2].y : y[u / 2].x) = v;
         (u & 1 ? go[u / 2].y : go[u / 2].x) = w;
@@ -593,8 +616,15 @@ static int px_update_go(const PairGeom& g, const float2* tw, const float2* S, co
     set_error("launch_x_inv_update", "partials buffer too small");
     return cudaErrorInvalidValue;
   }
-  auto kern = k_px_update<PL, NQ>;
-  const size_t smem = P::smem(0);
+  // Y and G come through shared memory where the arrays of an iteration do not
+  // stay in L2, which takes about 6 M voxels: the copies then run under the
+  // transform, where a prefetch into L2 leaves its latency to the walk.
+  // 108x324x525 takes 101 us against 111, 100x256x756 85.2 (Y alone) against
+  // 89.8, 64x500x1620 249 against 261; below it costs shared memory for
+  // nothing: 81x180x180 20.7 us against 18.9, 150x270x252 (10 M) 44.6 against 43.4.
+  const bool stage = Y && (long long)g.nx * g.ny * g.nz >= 12 << 20;
+  auto kern = stage ? k_px_update<PL, NQ, P::kStaged> : k_px_update<PL, NQ, 0>;
+  const size_t smem = P::smem(stage ? P::kStaged : 0);
   if (int rc = smem_optin(kern, smem)) return rc;
   float4* part = dots ? reinterpret_cast<float4*>(w->partials) : nullptr;
   const float* h0 = w ? w->h0 : nullptr;

@@ -79,3 +79,13 @@ def test_paired_ratio_outside_the_fast_range(cdx, oracle, torch_cuda, tmp_path):
     mine, fp64 = _rl(cdx, oracle, tmp_path, raw, 4)
     assert np.isfinite(mine).all()
     assert rel_l2(mine, fp64) < 5e-6
+
+
+def test_paired_rl_large_ragged_rows(cdx, oracle, torch_cuda, tmp_path):
+    """Rows of no whole 16-byte units in a volume past the L2 cache: the update
+    pass reads Y and G through shared memory there (an odd height leaves rows
+    of the last blocks empty).  Same bound as the smaller volumes'."""
+    raw = synth.bead_stack((98, 375, 350), n_beads=200, psf_sigma_xy=1.3, psf_sigma_z=2.0, seed=11)
+    mine, fp64 = _rl(cdx, oracle, tmp_path, raw, 3)
+    assert mine.shape == (98, 375, 350)
+    assert rel_l2(mine, fp64) < 5e-6
