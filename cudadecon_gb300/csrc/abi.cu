@@ -778,6 +778,7 @@ struct BatchStack {
   const unsigned short* h_raw = nullptr;
   float* h_result = nullptr;
   float background = 0.f;
+  cudaGraphNode_t up_node = nullptr, dn_node = nullptr;  // its copies in the graph
   void release() {
     plan.release();
     raw_otf.release();
@@ -804,6 +805,7 @@ struct Batch {
   cudaStream_t up = nullptr, dn = nullptr;
   cudaEvent_t ev_up = nullptr, ev_dn = nullptr, ev_jup = nullptr, ev_jdn = nullptr;
   cudaGraphExec_t exec = nullptr;
+  cudaGraph_t graph = nullptr;  // of exec, for its node handles
   int graph_iters = -1;
   int graph_form = -1;  // DFT form the graph's kernels were captured with
   int graph_host = -1;  // 1 when the graph carries the host transfers
@@ -812,7 +814,9 @@ struct Batch {
   long long last_launches = 0;
   void drop_graph() {
     if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
     exec = nullptr;
+    graph = nullptr;
     graph_iters = -1;
     graph_form = -1;
     graph_host = -1;
@@ -913,6 +917,34 @@ static int batch_setup_stack(BatchStack& b, const cdx_batch_stack& d, bool* chan
   return 0;
 }
 
+// The node that was captured last on stream s.
+static cudaError_t captured_node(cudaStream_t s, cudaGraphNode_t* node) {
+  cudaStreamCaptureStatus status;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t n = 0;
+  cudaError_t e = cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &deps, nullptr, &n);
+  if (e == cudaSuccess && (status != cudaStreamCaptureStatusActive || n != 1))
+    e = cudaErrorStreamCaptureInvalidated;
+  if (e == cudaSuccess) *node = deps[0];
+  return e;
+}
+
+// Point the captured copies of a stack at other host buffers.  A batch whose
+// buffers are new on every call would otherwise capture and instantiate its
+// graph each time: 4 of 9.7 ms for 12 stacks of up to 64x256x384.
+static bool batch_set_buffers(Batch& b, BatchStack& t, const unsigned short* raw, float* result) {
+  const float* src = b.graph_iters > 0 ? t.final_x : t.Xa.p;
+  const cudaError_t e1 = cudaGraphExecMemcpyNodeSetParams1D(
+      b.exec, t.up_node, t.u16.p, raw, sizeof(unsigned short) * (size_t)t.nx * t.ny * t.nz,
+      cudaMemcpyHostToDevice);
+  const cudaError_t e2 = cudaGraphExecMemcpyNodeSetParams1D(
+      b.exec, t.dn_node, result, src, sizeof(float) * (size_t)t.gx * t.gy * t.gz,
+      cudaMemcpyDeviceToHost);
+  if (e1 == cudaSuccess && e2 == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+
 // Capture the iterations of every stack into b.exec; with host, each
 // stack's chain also conditions its raw stack first, after its upload on
 // the upload stream, and its result is downloaded on the download stream
@@ -954,6 +986,7 @@ static int batch_capture(Batch& b, int nIters, bool host) {
       const size_t nin = (size_t)t.nx * t.ny * t.nz;
       if ((e = cudaMemcpyAsync(t.u16.p, t.h_raw, nin * sizeof(unsigned short),
                                cudaMemcpyHostToDevice, b.up)) != cudaSuccess ||
+          (e = captured_node(b.up, &t.up_node)) != cudaSuccess ||
           (e = cudaEventRecord(b.ev_up, b.up)) != cudaSuccess ||
           (e = cudaStreamWaitEvent(s, b.ev_up, 0)) != cudaSuccess) {
         set_cuda_error("batch capture", e);
@@ -982,7 +1015,8 @@ static int batch_capture(Batch& b, int nIters, bool host) {
       if ((e = cudaEventRecord(b.ev_dn, s)) != cudaSuccess ||
           (e = cudaStreamWaitEvent(b.dn, b.ev_dn, 0)) != cudaSuccess ||
           (e = cudaMemcpyAsync(t.h_result, src, n * sizeof(float), cudaMemcpyDeviceToHost,
-                               b.dn)) != cudaSuccess) {
+                               b.dn)) != cudaSuccess ||
+          (e = captured_node(b.dn, &t.dn_node)) != cudaSuccess) {
         set_cuda_error("batch capture", e);
         rc = e;
       }
@@ -1018,11 +1052,12 @@ static int batch_capture(Batch& b, int nIters, bool host) {
       rc = e;
     }
   }
-  if (graph) cudaGraphDestroy(graph);
   if (rc) {
+    if (graph) cudaGraphDestroy(graph);
     cudaGetLastError();
     return rc;
   }
+  b.graph = graph;
   b.graph_iters = nIters;
   b.graph_form = dft_form();
   b.graph_host = host ? 1 : 0;
@@ -1078,12 +1113,14 @@ static int batch_run(const cdx_batch_stack* stacks, int n, int nIters, cudaStrea
   }
   if (changed) b.drop_graph();
   if (host) {
-    // the graph bakes in the host buffers and backgrounds
+    // the graph holds the host buffers and backgrounds
     for (int i = 0; i < n; ++i) {
       BatchStack& t = b.st[i];
       const cdx_batch_stack& d = stacks[i];
       if ((rc = t.u16.ensure((size_t)d.nx * d.ny * d.nz))) return rc;
-      if (t.h_raw != d.raw || t.h_result != d.result || t.background != d.background)
+      const bool moved = t.h_raw != d.raw || t.h_result != d.result;
+      if (t.background != d.background) b.drop_graph();
+      else if (moved && b.exec && b.graph_host == 1 && !batch_set_buffers(b, t, d.raw, d.result))
         b.drop_graph();
       t.h_raw = d.raw;
       t.h_result = d.result;
