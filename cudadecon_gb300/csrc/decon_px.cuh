@@ -248,7 +248,7 @@ __device__ __forceinline__ void spec_to_tile(const PairGeom& g, float4* sm, cons
 template <class PL, int NQ>
 __global__ void __launch_bounds__(PX<PL, NQ>::T, PX<PL, NQ>::kBlocksFwd)
 k_px_fwd(PairGeom g, const float2* __restrict__ tw, const float* X, float* Xm1, const float* lamp,
-         int predict, float4* S) {
+         int predict, float bg, float4* S) {
   using P = PX<PL, NQ>;
   extern __shared__ __align__(16) float2 smem[];
   float2* stw = smem;
@@ -284,6 +284,10 @@ k_px_fwd(PairGeom g, const float2* __restrict__ tw, const float* X, float* Xm1, 
         x[r].im = relu2(fma2(lam, sub2(x[r].im, o.im), x[r].im));
         st_rows<true>(pm + r * PL::KC, rq, PL::L, x[r]);
       }
+    } else if (bg != 0.f) {  // rows past the volume stay 0
+      const float2 im = make_float2(rq.v2 ? -bg : 0.f, rq.v3 ? -bg : 0.f);
+#pragma unroll
+      for (int r = 0; r < PL::Q2; ++r) x[r] = {add2(x[r].re, dup2(-bg)), add2(x[r].im, im)};
     }
   } else {
 #pragma unroll
@@ -581,13 +585,13 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
 // ---------------------------------------------------------------- launches
 template <class PL, int NQ>
 static int px_fwd_go(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
-                     const float* lam, int predict, float2* S, cudaStream_t st) {
+                     const float* lam, int predict, float bg, float2* S, cudaStream_t st) {
   using P = PX<PL, NQ>;
   auto kern = k_px_fwd<PL, NQ>;
   const size_t smem = P::smem_fwd(predict ? 2 : 1);
   if (int rc = smem_optin(kern, smem)) return rc;
   CDX_CHECK(launch_pdl(kern, dim3(ceil_div(g.H / 2, NQ), g.nz), dim3(P::T), smem, st, g, tw, X,
-                       Xm1, lam, predict, reinterpret_cast<float4*>(S)));
+                       Xm1, lam, predict, bg, reinterpret_cast<float4*>(S)));
   CDX_LAUNCH_CHECK("k_px_fwd");
   return 0;
 }

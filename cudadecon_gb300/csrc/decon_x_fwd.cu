@@ -8,12 +8,16 @@
 namespace cdx {
 
 int launch_x_fwd(const Geom& g, const FftLen& fx, const float* X, float* Xm1,
-                 const float* lam, int predict, float2* S, cudaStream_t st) {
+                 const float* lam, int predict, float2* S, cudaStream_t st, float bg) {
+  if (bg != 0.f && (!g.pair || predict)) {
+    set_error("launch_x_fwd", "a background is subtracted by the paired pass without prediction");
+    return cudaErrorInvalidValue;
+  }
   if (!g.pair && fx.has_tc && dft_form() == 1)
     return launch_xtc_fwd(g, fx.tc, X, Xm1, lam, predict, S, fx.tc.d_err, st);
   if (g.pair) {
     bool done = false;
-    const int rc = pxgen_fwd(pair_geom(g), fx.d_pair, X, Xm1, lam, predict, S, st, &done);
+    const int rc = pxgen_fwd(pair_geom(g), fx.d_pair, X, Xm1, lam, predict, bg, S, st, &done);
     if (done || rc) return rc;
   }
   const int P = x_pairs(g.nx);

@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_0(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_0(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 128:
       *done = true;
-      return px_fwd_go<PPX128, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX128, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 243:
       *done = true;
-      return px_fwd_go<PPX243, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX243, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 392:
       *done = true;
-      return px_fwd_go<PPX392, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX392, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 600:
       *done = true;
-      return px_fwd_go<PPX600, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX600, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 875:
       *done = true;
-      return px_fwd_go<PPX875, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX875, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1215:
       *done = true;
-      return px_fwd_go<PPX1215, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1215, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1620:
       *done = true;
-      return px_fwd_go<PPX1620, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1620, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

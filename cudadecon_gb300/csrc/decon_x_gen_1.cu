@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_1(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_1(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 135:
       *done = true;
-      return px_fwd_go<PPX135, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX135, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 245:
       *done = true;
-      return px_fwd_go<PPX245, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX245, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 400:
       *done = true;
-      return px_fwd_go<PPX400, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX400, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 625:
       *done = true;
-      return px_fwd_go<PPX625, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX625, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 882:
       *done = true;
-      return px_fwd_go<PPX882, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX882, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1225:
       *done = true;
-      return px_fwd_go<PPX1225, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1225, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1680:
       *done = true;
-      return px_fwd_go<PPX1680, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1680, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

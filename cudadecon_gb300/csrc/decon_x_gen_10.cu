@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_10(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_10(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 180:
       *done = true;
-      return px_fwd_go<PPX180, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX180, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 315:
       *done = true;
-      return px_fwd_go<PPX315, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX315, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 490:
       *done = true;
-      return px_fwd_go<PPX490, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX490, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 729:
       *done = true;
-      return px_fwd_go<PPX729, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX729, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1024:
       *done = true;
-      return px_fwd_go<PPX1024, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1024, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1400:
       *done = true;
-      return px_fwd_go<PPX1400, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1400, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1920:
       *done = true;
-      return px_fwd_go<PPX1920, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1920, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_11(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_11(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 189:
       *done = true;
-      return px_fwd_go<PPX189, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX189, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 320:
       *done = true;
-      return px_fwd_go<PPX320, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX320, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 500:
       *done = true;
-      return px_fwd_go<PPX500, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX500, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 735:
       *done = true;
-      return px_fwd_go<PPX735, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX735, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1029:
       *done = true;
-      return px_fwd_go<PPX1029, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1029, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1440:
       *done = true;
-      return px_fwd_go<PPX1440, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1440, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1944:
       *done = true;
-      return px_fwd_go<PPX1944, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1944, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_12(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_12(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 192:
       *done = true;
-      return px_fwd_go<PPX192, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX192, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 324:
       *done = true;
-      return px_fwd_go<PPX324, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX324, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 504:
       *done = true;
-      return px_fwd_go<PPX504, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX504, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 750:
       *done = true;
-      return px_fwd_go<PPX750, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX750, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1050:
       *done = true;
-      return px_fwd_go<PPX1050, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1050, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1458:
       *done = true;
-      return px_fwd_go<PPX1458, 4>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1458, 4>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1960:
       *done = true;
-      return px_fwd_go<PPX1960, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1960, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_13(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_13(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 196:
       *done = true;
-      return px_fwd_go<PPX196, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX196, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 336:
       *done = true;
-      return px_fwd_go<PPX336, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX336, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 512:
       *done = true;
-      return px_fwd_go<PPX512, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX512, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 756:
       *done = true;
-      return px_fwd_go<PPX756, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX756, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1080:
       *done = true;
-      return px_fwd_go<PPX1080, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1080, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1470:
       *done = true;
-      return px_fwd_go<PPX1470, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1470, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 2000:
       *done = true;
-      return px_fwd_go<PPX2000, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX2000, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_14(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_14(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 200:
       *done = true;
-      return px_fwd_go<PPX200, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX200, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 343:
       *done = true;
-      return px_fwd_go<PPX343, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX343, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 525:
       *done = true;
-      return px_fwd_go<PPX525, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX525, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 768:
       *done = true;
-      return px_fwd_go<PPX768, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX768, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1120:
       *done = true;
-      return px_fwd_go<PPX1120, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1120, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1500:
       *done = true;
-      return px_fwd_go<PPX1500, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1500, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 2016:
       *done = true;
-      return px_fwd_go<PPX2016, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX2016, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_15(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_15(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 210:
       *done = true;
-      return px_fwd_go<PPX210, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX210, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 350:
       *done = true;
-      return px_fwd_go<PPX350, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX350, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 540:
       *done = true;
-      return px_fwd_go<PPX540, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX540, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 784:
       *done = true;
-      return px_fwd_go<PPX784, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX784, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1125:
       *done = true;
-      return px_fwd_go<PPX1125, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1125, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1512:
       *done = true;
-      return px_fwd_go<PPX1512, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1512, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 2025:
       *done = true;
-      return px_fwd_go<PPX2025, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX2025, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

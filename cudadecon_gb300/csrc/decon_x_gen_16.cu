@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_16(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_16(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 216:
       *done = true;
-      return px_fwd_go<PPX216, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX216, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 360:
       *done = true;
-      return px_fwd_go<PPX360, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX360, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 560:
       *done = true;
-      return px_fwd_go<PPX560, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX560, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 800:
       *done = true;
-      return px_fwd_go<PPX800, 4>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX800, 4>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1134:
       *done = true;
-      return px_fwd_go<PPX1134, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1134, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1536:
       *done = true;
-      return px_fwd_go<PPX1536, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1536, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 2048:
       *done = true;
-      return px_fwd_go<PPX2048, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX2048, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

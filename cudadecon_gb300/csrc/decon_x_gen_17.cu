@@ -6,26 +6,26 @@
 
 namespace cdx {
 
-int pxgen_fwd_17(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_17(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 224:
       *done = true;
-      return px_fwd_go<PPX224, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX224, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 375:
       *done = true;
-      return px_fwd_go<PPX375, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX375, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 567:
       *done = true;
-      return px_fwd_go<PPX567, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX567, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 810:
       *done = true;
-      return px_fwd_go<PPX810, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX810, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1152:
       *done = true;
-      return px_fwd_go<PPX1152, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1152, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1568:
       *done = true;
-      return px_fwd_go<PPX1568, 4>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1568, 4>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

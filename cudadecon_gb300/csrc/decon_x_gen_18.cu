@@ -6,26 +6,26 @@
 
 namespace cdx {
 
-int pxgen_fwd_18(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_18(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 225:
       *done = true;
-      return px_fwd_go<PPX225, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX225, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 378:
       *done = true;
-      return px_fwd_go<PPX378, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX378, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 576:
       *done = true;
-      return px_fwd_go<PPX576, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX576, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 840:
       *done = true;
-      return px_fwd_go<PPX840, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX840, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1176:
       *done = true;
-      return px_fwd_go<PPX1176, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1176, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1575:
       *done = true;
-      return px_fwd_go<PPX1575, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1575, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

@@ -6,26 +6,26 @@
 
 namespace cdx {
 
-int pxgen_fwd_19(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_19(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 240:
       *done = true;
-      return px_fwd_go<PPX240, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX240, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 384:
       *done = true;
-      return px_fwd_go<PPX384, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX384, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 588:
       *done = true;
-      return px_fwd_go<PPX588, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX588, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 864:
       *done = true;
-      return px_fwd_go<PPX864, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX864, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1200:
       *done = true;
-      return px_fwd_go<PPX1200, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1200, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1600:
       *done = true;
-      return px_fwd_go<PPX1600, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1600, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_2(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_2(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 140:
       *done = true;
-      return px_fwd_go<PPX140, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX140, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 250:
       *done = true;
-      return px_fwd_go<PPX250, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX250, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 405:
       *done = true;
-      return px_fwd_go<PPX405, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX405, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 630:
       *done = true;
-      return px_fwd_go<PPX630, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX630, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 896:
       *done = true;
-      return px_fwd_go<PPX896, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX896, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1250:
       *done = true;
-      return px_fwd_go<PPX1250, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1250, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1701:
       *done = true;
-      return px_fwd_go<PPX1701, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1701, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_3(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_3(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 144:
       *done = true;
-      return px_fwd_go<PPX144, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX144, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 252:
       *done = true;
-      return px_fwd_go<PPX252, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX252, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 420:
       *done = true;
-      return px_fwd_go<PPX420, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX420, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 640:
       *done = true;
-      return px_fwd_go<PPX640, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX640, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 900:
       *done = true;
-      return px_fwd_go<PPX900, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX900, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1260:
       *done = true;
-      return px_fwd_go<PPX1260, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1260, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1728:
       *done = true;
-      return px_fwd_go<PPX1728, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1728, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

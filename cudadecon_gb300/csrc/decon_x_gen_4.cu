@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_4(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_4(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 147:
       *done = true;
-      return px_fwd_go<PPX147, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX147, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 256:
       *done = true;
-      return px_fwd_go<PPX256, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX256, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 432:
       *done = true;
-      return px_fwd_go<PPX432, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX432, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 648:
       *done = true;
-      return px_fwd_go<PPX648, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX648, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 945:
       *done = true;
-      return px_fwd_go<PPX945, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX945, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1280:
       *done = true;
-      return px_fwd_go<PPX1280, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1280, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1750:
       *done = true;
-      return px_fwd_go<PPX1750, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1750, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

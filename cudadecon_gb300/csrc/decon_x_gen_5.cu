@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_5(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_5(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 150:
       *done = true;
-      return px_fwd_go<PPX150, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX150, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 270:
       *done = true;
-      return px_fwd_go<PPX270, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX270, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 441:
       *done = true;
-      return px_fwd_go<PPX441, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX441, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 672:
       *done = true;
-      return px_fwd_go<PPX672, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX672, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 960:
       *done = true;
-      return px_fwd_go<PPX960, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX960, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1296:
       *done = true;
-      return px_fwd_go<PPX1296, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1296, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1764:
       *done = true;
-      return px_fwd_go<PPX1764, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1764, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

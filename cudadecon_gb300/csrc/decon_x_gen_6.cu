@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_6(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_6(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 160:
       *done = true;
-      return px_fwd_go<PPX160, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX160, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 280:
       *done = true;
-      return px_fwd_go<PPX280, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX280, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 448:
       *done = true;
-      return px_fwd_go<PPX448, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX448, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 675:
       *done = true;
-      return px_fwd_go<PPX675, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX675, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 972:
       *done = true;
-      return px_fwd_go<PPX972, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX972, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1323:
       *done = true;
-      return px_fwd_go<PPX1323, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1323, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1792:
       *done = true;
-      return px_fwd_go<PPX1792, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1792, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

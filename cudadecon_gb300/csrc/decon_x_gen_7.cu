@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_7(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_7(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 162:
       *done = true;
-      return px_fwd_go<PPX162, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX162, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 288:
       *done = true;
-      return px_fwd_go<PPX288, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX288, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 450:
       *done = true;
-      return px_fwd_go<PPX450, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX450, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 686:
       *done = true;
-      return px_fwd_go<PPX686, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX686, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 980:
       *done = true;
-      return px_fwd_go<PPX980, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX980, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1344:
       *done = true;
-      return px_fwd_go<PPX1344, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1344, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1800:
       *done = true;
-      return px_fwd_go<PPX1800, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1800, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

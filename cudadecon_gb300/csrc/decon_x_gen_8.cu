@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_8(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_8(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 168:
       *done = true;
-      return px_fwd_go<PPX168, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX168, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 294:
       *done = true;
-      return px_fwd_go<PPX294, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX294, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 480:
       *done = true;
-      return px_fwd_go<PPX480, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX480, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 700:
       *done = true;
-      return px_fwd_go<PPX700, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX700, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1000:
       *done = true;
-      return px_fwd_go<PPX1000, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1000, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1350:
       *done = true;
-      return px_fwd_go<PPX1350, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1350, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1875:
       *done = true;
-      return px_fwd_go<PPX1875, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1875, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

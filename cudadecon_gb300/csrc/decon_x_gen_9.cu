@@ -6,29 +6,29 @@
 
 namespace cdx {
 
-int pxgen_fwd_9(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+int pxgen_fwd_9(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 175:
       *done = true;
-      return px_fwd_go<PPX175, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX175, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 300:
       *done = true;
-      return px_fwd_go<PPX300, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX300, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 486:
       *done = true;
-      return px_fwd_go<PPX486, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX486, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 720:
       *done = true;
-      return px_fwd_go<PPX720, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX720, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1008:
       *done = true;
-      return px_fwd_go<PPX1008, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1008, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1372:
       *done = true;
-      return px_fwd_go<PPX1372, 4>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1372, 4>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1890:
       *done = true;
-      return px_fwd_go<PPX1890, 2>(g, tw, X, Xm1, lam, predict, S, st);
+      return px_fwd_go<PPX1890, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     default:
       return 0;
   }

@@ -122,9 +122,10 @@ struct RLWork {
 int x_pass_blocks(const Geom& g);
 // Forward x pass: Y (from X, Xm1, lambda when predict != 0, else Y = X) ->
 // spectrum after the R2C along x.  When predict != 0, Y = max(X + lam*(X - Xm1), 0)
-// is also written over Xm1 (whose old values are not needed afterwards).
+// is also written over Xm1 (whose old values are not needed afterwards).  bg is
+// subtracted from X (paired layout without prediction only).
 int launch_x_fwd(const Geom& g, const FftLen& fx, const float* X, float* Xm1,
-                 const float* lam, int predict, float2* S, cudaStream_t st);
+                 const float* lam, int predict, float2* S, cudaStream_t st, float bg = 0.f);
 // In-place complex FFT along y of every (kx, z) row.
 int launch_y_pass(const Geom& g, const FftLen& fy, float2* S, bool inverse, cudaStream_t st);
 // z FFT, multiply by OTF (or its conjugate), inverse z FFT, in place.

@@ -7,26 +7,26 @@
 
 namespace cdx {
 
-int pxgen_fwd_0(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_1(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_2(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_3(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_4(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_5(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_6(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_7(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_8(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_9(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_10(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_11(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_12(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_13(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_14(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_15(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_16(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_17(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_18(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
-int pxgen_fwd_19(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_0(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_1(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_2(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_3(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_4(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_5(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_6(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_7(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_8(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_9(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_10(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_11(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_12(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_13(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_14(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_15(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_16(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_17(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_18(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
+int pxgen_fwd_19(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
 int pxgen_ratio_0(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
 int pxgen_ratio_1(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
 int pxgen_ratio_2(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
@@ -84,29 +84,29 @@ int pzgen_5(const PairGeom& g, const float2* tw, float2* S, const OtfDev& otf, b
 int pzgen_6(const PairGeom& g, const float2* tw, float2* S, const OtfDev& otf, bool conj, cudaStream_t st, bool fwd_only, bool* done);
 int pzgen_7(const PairGeom& g, const float2* tw, float2* S, const OtfDev& otf, bool conj, cudaStream_t st, bool fwd_only, bool* done);
 
-inline int pxgen_fwd(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float2* S, cudaStream_t st, bool* done) {
+inline int pxgen_fwd(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done) {
   int rc = 0;
   *done = false;
-  if ((rc = pxgen_fwd_0(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_1(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_2(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_3(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_4(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_5(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_6(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_7(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_8(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_9(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_10(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_11(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_12(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_13(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_14(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_15(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_16(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_17(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_18(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
-  if ((rc = pxgen_fwd_19(g, tw, X, Xm1, lam, predict, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_0(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_1(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_2(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_3(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_4(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_5(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_6(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_7(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_8(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_9(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_10(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_11(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_12(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_13(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_14(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_15(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_16(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_17(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_18(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
+  if ((rc = pxgen_fwd_19(g, tw, X, Xm1, lam, predict, bg, S, st, done)) || *done) return rc;
   return 0;
 }
 
