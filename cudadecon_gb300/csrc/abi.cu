@@ -749,7 +749,8 @@ static int init_session(Session& s, int nx, int ny, int nz, float dr, float dz, 
 // the stacks, largest first, each go to the least-loaded of K streams forked
 // from the origin stream, so the graph holds K independent chains of about
 // equal work and small stacks run concurrently.  K is 2 by default
-// (cdx_batch_set_streams): on the 64-stack uneven batch, device-resident,
+// (cdx_batch_set_streams): on the 64-stack uneven batch, device-resident and
+// with the unpaired passes,
 // 1, 2, 3, 4, 6, 8 and 16 streams gave 42.7, 44.6, 43.9, 42.6, 40.2, 39.9 and
 // 39.9 G voxel-iter/s (more concurrent stacks share the L2 that holds a
 // stack's spectrum between its passes).  The host batch's transfers run on
@@ -773,7 +774,7 @@ struct BatchStack {
   DevBuf<float> lam;
   float* final_x = nullptr;
   // host mode (cdx_RL_batch_host): the stack's device copy of the caller's
-  // page-locked raw buffer, and what the captured graph baked in
+  // page-locked raw buffer, and what the captured graph holds
   DevBuf<unsigned short> u16;
   const unsigned short* h_raw = nullptr;
   float* h_result = nullptr;

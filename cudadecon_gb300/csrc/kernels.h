@@ -6,13 +6,6 @@
 
 namespace cdx {
 
-// Geometry of one real volume (x fastest) and of its half spectrum.
-//
-// The spectrum is an internal buffer and uses kx-plane-major order
-// S[kx][z][y] (y fastest, row pitch nyp = ny rounded up to even), unlike
-// cuFFT's [z][y][kx].  Each plane holds the (z, y) samples of one kx column,
-// so the y pass reads contiguous rows, the z pass reads 128-byte runs, and
-// the x passes write and read transposed 16-byte (two-row) groups.
 // The paired layout (pair_layout.cuh) at height ny: which row shares a complex
 // row with row y (y + pair_split), and the slots per half row.
 __host__ __device__ inline constexpr int pair_split(int ny) {
@@ -20,6 +13,14 @@ __host__ __device__ inline constexpr int pair_split(int ny) {
 }
 __host__ __device__ inline constexpr int pair_half(int ny) { return (pair_split(ny) / 2 + 3) / 4 * 4; }
 
+// Geometry of one real volume (x fastest) and of its half spectrum.
+//
+// The spectrum is an internal buffer, in the paired layout (pair_layout.cuh) or,
+// where a grid has no paired passes, in kx-plane-major order
+// S[kx][z][y] (y fastest, row pitch nyp = ny rounded up to even), unlike
+// cuFFT's [z][y][kx].  Each plane holds the (z, y) samples of one kx column,
+// so the y pass reads contiguous rows, the z pass reads 128-byte runs, and
+// the x passes write and read transposed 16-byte (two-row) groups.
 struct Geom {
   int nx, ny, nz;
   int nxh;         // nx/2 + 1

@@ -23,7 +23,9 @@ between the stages); candidate 0 is the heuristic choice:
          radices (the most balanced triple) with the full and half batch:
          an unbalanced pair such as 125 = 25*5 leaves most threads idle in
          its large-radix stage.
-  x    : the most balanced three radices, smallest last (the fused epilogues
+  x    : (chosen and tuned, but compiled into nothing: the paired passes took
+         over every x length of a plan)
+         the most balanced three radices, smallest last (the fused epilogues
          of the x passes run in the last stage, which then has a thread for
          every butterfly), with the generic engine's row pairs per block.
          Candidates: half the row pairs, the two larger radices swapped, the
