@@ -38,7 +38,10 @@ void set_error(const char* where, const char* what) {
   g_err_shared = s;
 }
 
-void set_cuda_error(const char* where, cudaError_t err) { set_error(where, cudaGetErrorString(err)); }
+void set_cuda_error(const char* where, cudaError_t err) {
+  cudaGetLastError();  // reported here: the next call's launch check must not find it
+  set_error(where, cudaGetErrorString(err));
+}
 
 // ---------------------------------------------------------------- sizes
 // Good FFT sizes are products of 2, 3, 5 and 7 (notGoodDimension /

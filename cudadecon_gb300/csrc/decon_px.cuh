@@ -165,13 +165,14 @@ struct PX {
   static constexpr int kBlocksFwd = resident_blocks(by_regs(24 + 4 * PL::qmax()), smem_fwd(2));
   static constexpr int kRegsUpd = 24 + 4 * PL::qmax() > 64 ? 24 + 4 * PL::qmax() : 64;
   // Row arrays (Y, then G) that the update pass of a large volume has in shared
-  // memory: as many as leave 512 threads an SM, or all that fit beside the
-  // blocks there are without them.  One block of two lost 27% of the pass at 800
-  // columns, two of four (448 threads) 9% at 756, three of eight (192) 13% at
-  // 625; three of four (672) gained 6% at 700, four of eight (512) 3% at 512.
+  // memory: as many as fit a block and leave 512 threads an SM, or all that fit
+  // beside the blocks there are without them.  One block of two lost 27% of the
+  // pass at 800 columns, two of four (448 threads) 9% at 756, three of eight
+  // (192) 13% at 625; three of four (672) gained 6% at 700, four of eight (512)
+  // 3% at 512.  Against the rule 567 (+3%) and 980 (+1.6% of the pass) lost.
   static constexpr int blocks_upd(int R) { return resident_blocks(by_regs(kRegsUpd), smem(R)); }
   static constexpr bool stages(int R) {
-    return blocks_upd(R) * T >= 512 || blocks_upd(R) == blocks_upd(0);
+    return blocks_upd(R) > 0 && (blocks_upd(R) * T >= 512 || blocks_upd(R) == blocks_upd(0));
   }
   static constexpr int kStaged = stages(2) ? 2 : (stages(1) ? 1 : 0);
   __device__ __forceinline__ static float* rows_fwd(float2* sm, int i) {
@@ -587,6 +588,7 @@ template <class PL, int NQ>
 static int px_fwd_go(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
                      const float* lam, int predict, float bg, float2* S, cudaStream_t st) {
   using P = PX<PL, NQ>;
+  static_assert(P::kBlocksFwd > 0, "an SM holds a block");
   auto kern = k_px_fwd<PL, NQ>;
   const size_t smem = P::smem_fwd(predict ? 2 : 1);
   if (int rc = smem_optin(kern, smem)) return rc;
@@ -600,6 +602,7 @@ template <class PL, int NQ>
 static int px_ratio_go(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps,
                        cudaStream_t st) {
   using P = PX<PL, NQ>;
+  static_assert(P::kBlocks > 0, "an SM holds a block");
   auto kern = k_px_ratio<PL, NQ>;
   const size_t smem = P::smem(1);
   if (int rc = smem_optin(kern, smem)) return rc;
@@ -614,6 +617,7 @@ static int px_update_go(const PairGeom& g, const float2* tw, const float2* S, co
                         float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps,
                         cudaStream_t st) {
   using P = PX<PL, NQ>;
+  static_assert(P::blocks_upd(0) > 0 && P::blocks_upd(P::kStaged) > 0, "an SM holds a block");
   const dim3 grid(ceil_div(g.H / 2, NQ), g.nz);
   const int nblk = grid.x * grid.y;
   if (dots && nblk > w->max_blocks) {

@@ -22,7 +22,7 @@ struct PZ {
   static constexpr int kTile = W * PL::L;  // float4s
   static constexpr size_t kSmem = sizeof(float2) * kTw + 2 * sizeof(float4) * kTile;
   static constexpr int kBlocks = resident_blocks(PL::blocks(W, 56 /*Z*/), kSmem);
-  static_assert(T % W == 0, "a thread copies one column");
+  static_assert(T % W == 0 && kBlocks > 0, "a thread copies one column, an SM holds a block");
 };
 
 // MODE 0: radially averaged table (CONJ: its conjugate); 1: full 3D array in

@@ -267,11 +267,12 @@ __device__ __forceinline__ void copy_twiddles(const float2* tw, float2* stw) {
   for (int i = threadIdx.x; i < N / 2; i += blockDim.x) cp_async16(stw + 2 * i, tw + 2 * i);
 }
 
-// Blocks per SM of a kernel that walks over tiles: the launch bound, or what
-// the shared memory of an SM (227 KB, 1 KB of it reserved per block) holds.
+// Blocks per SM: the launch bound, or what the shared memory of an SM (227 KB,
+// 1 KB of it kept per block, which covers the kernels' static arrays) holds; 0
+// where not even one block fits.
 constexpr int resident_blocks(int bound, size_t smem) {
   const int fit = (int)((227u << 10) / (smem + 1024));
-  return fit < 1 ? 1 : (fit < bound ? fit : bound);
+  return fit < bound ? fit : bound;
 }
 
 // Twiddle factors in the layout of FftDev::tw (stage with span Ns at Ns - 1,
