@@ -61,7 +61,7 @@ static bool factorize(int L, std::vector<int>& rad) {
   while (n % 5 == 0) { rad.push_back(5); n /= 5; }
   if (n != 1) return false;
   if ((int)rad.size() > kMaxStages) return false;
-  if (rad.empty()) rad.push_back(1);  // L == 1: identity
+  if (rad.empty()) rad.push_back(1);  // L == 1: identity, a copy from loader to storer
   return true;
 }
 
@@ -75,7 +75,7 @@ bool fft_len_supported(int L) {
 // [Ns-1 + (r-1)*Ns + k], computed in double and rounded once to float.
 static int build_fft_dev(int L, const std::vector<int>& rad, FftDev& d, float2** d_tw) {
   d.L = L;
-  d.nst = (rad.size() == 1 && rad[0] == 1) ? 0 : (int)rad.size();
+  d.nst = (int)rad.size();  // a length of 1 has one stage of radix 1
   std::vector<float2> tw(L, make_float2(1.f, 0.f));
   const double two_pi = 6.283185307179586476925286766559;
   int Ns = 1;

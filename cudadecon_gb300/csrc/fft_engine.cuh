@@ -120,6 +120,11 @@ template <int R, bool INV>
 struct Dft;
 
 template <bool INV>
+struct Dft<1, INV> {  // the only stage of a length of 1
+  __host__ __device__ __forceinline__ static void run(float2*) {}
+};
+
+template <bool INV>
 struct Dft<2, INV> {
   __host__ __device__ __forceinline__ static void run(float2* x) {
     float2 a = x[0], b = x[1];
@@ -375,6 +380,7 @@ template <bool INV, bool SYNC_MID, bool SYNC_END, class Ld, class St>
 __device__ __forceinline__ void stage_any(const StageDev& sd, int V, float invV, bool vfast,
                                           const float2* stw, const Ld& ld, const St& st) {
   switch (sd.R) {
+    case 1: stage_io<1, INV, SYNC_MID, SYNC_END>(sd, V, invV, vfast, stw, ld, st); break;
     case 2: stage_io<2, INV, SYNC_MID, SYNC_END>(sd, V, invV, vfast, stw, ld, st); break;
     case 3: stage_io<3, INV, SYNC_MID, SYNC_END>(sd, V, invV, vfast, stw, ld, st); break;
     case 4: stage_io<4, INV, SYNC_MID, SYNC_END>(sd, V, invV, vfast, stw, ld, st); break;
