@@ -189,7 +189,7 @@ void choose_layout(Geom& g, const FftLen& fx, const FftLen& fy) {
   const bool z_fits = 2 * g.nz <= kMaxThreads * kEpt;
   // slot offsets within a slice are 32-bit
   const bool s_fits = (long long)pair_half(g.ny) * 2 * g.nxh < (1LL << 31);
-  g.pair = fx.d_pair && z_fits && s_fits && !(dft_form() == 1 && fx.has_tc);
+  g.pair = fx.d_pair && z_fits && s_fits && pair_rows(g.ny) && !(dft_form() == 1 && fx.has_tc);
   g.eo = g.pair && fy.d_pair && fy.pair_eo;
 }
 

@@ -11,6 +11,9 @@ namespace cdx {
 __host__ __device__ inline constexpr int pair_split(int ny) {
   return ny < 4 ? 2 : ny % 4 == 0 ? ny / 2 : ((ny + 1) / 2 + 3) / 4 * 4;
 }
+// Whether both rows of a slot's first half exist in all its slots: a height of 1
+// has only the first (its second would be the next slice's row).
+__host__ __device__ inline constexpr bool pair_rows(int ny) { return pair_split(ny) <= ny; }
 __host__ __device__ inline constexpr int pair_half(int ny) { return (pair_split(ny) / 2 + 3) / 4 * 4; }
 
 // Geometry of one real volume (x fastest) and of its half spectrum.
