@@ -35,7 +35,7 @@ k_x_fwd(Geom g, FftDev fx, const float* __restrict__ X, float* Xm1, const float*
   prefetch_floats(Xs, X + roff, nr * nx, true);
   if (predict) prefetch_floats(Xm1s, Xm1 + roff, nr * nx, true);
   cp_async_commit();
-  const float lam = predict ? __ldg(lamp) : 0.f;
+  const float lam = predict ? __ldcg(lamp) : 0.f;
   cp_async_wait_all();
   __syncthreads();
   // prediction of updatePrediction_kernel (RLgpuImpl.cu:658-666), applied
