@@ -380,8 +380,8 @@ static int ensure_grid_buffers(Session& s, const Geom& g) {
       (rc = s.raw.ensure(n)) || (rc = s.S.ensure((size_t)g.spec_elems())))
     return rc;
   const int nblk = x_pass_blocks(g);
-  if ((rc = s.partials.ensure(2 * (size_t)nblk)) || (rc = s.lam.ensure(2))) return rc;
-  CDX_CHECK(cudaMemsetAsync(s.lam.p, 0, 2 * sizeof(float), s.stream));
+  if ((rc = s.partials.ensure(2 * (size_t)nblk)) || (rc = s.lam.ensure(4))) return rc;
+  CDX_CHECK(cudaMemsetAsync(s.lam.p, 0, 4 * sizeof(float), s.stream));
   return 0;
 }
 
@@ -390,7 +390,8 @@ static int ensure_grid_buffers(Session& s, const Geom& g) {
 // the grid of s.plan, starting from X0 in s.Xa with raw in s.raw.  Returns
 // the buffer that holds the final estimate.
 // Device buffers of one RL loop: estimates (X0 in Xa), raw, G, spectrum,
-// dot-product partials (16 bytes per x-pass block) and the two lambda slots.
+// dot-product partials (16 bytes per x-pass block), two lambda slots and, behind
+// them, two for the mean of the ratio.
 struct LoopBufs {
   float* Xa;
   float* Xb;
@@ -412,6 +413,8 @@ static int rl_loop(const GridPlan& p, const LoopBufs& b, int nIter, cudaStream_t
   w.lam = b.lam;
   w.max_blocks = b.max_blocks;
   w.h0 = p.otf.h0;
+  OtfDev conj = p.otf;  // second convolution: keeps the ratio's mean as it passes
+  conj.inv2n = (float)(0.5 / (double)g.nvox());
   const float eps = 1.1920928955078125e-07f;  // std::numeric_limits<float>::epsilon()
   float* X = b.Xa;
   float* Xm1 = b.Xb;
@@ -435,11 +438,14 @@ static int rl_loop(const GridPlan& p, const LoopBufs& b, int nIter, cudaStream_t
     mark();
     if ((rc = launch_y_pass(g, p.fy, b.S, true, st))) return rc;
     mark();
-    if ((rc = launch_x_inv_ratio_fwd(g, p.fx, b.S, b.raw, eps, st))) return rc;
+    // the mean of the last iteration's ratio is taken off this one's
+    w.mean = conj.mean = k > 0 ? b.lam + 2 + (k & 1) : nullptr;
+    conj.mean_next = b.lam + 2 + ((k + 1) & 1);
+    if ((rc = launch_x_inv_ratio_fwd(g, p.fx, b.S, b.raw, w.mean, eps, st))) return rc;
     mark();
     if ((rc = launch_y_pass(g, p.fy, b.S, false, st))) return rc;
     mark();
-    if ((rc = launch_z_pass(g, p.fz, b.S, p.otf, true, st))) return rc;
+    if ((rc = launch_z_pass(g, p.fz, b.S, conj, true, st))) return rc;
     mark();
     if ((rc = launch_y_pass(g, p.fy, b.S, true, st))) return rc;
     mark();
@@ -915,7 +921,7 @@ static int batch_setup_stack(BatchStack& b, const cdx_batch_stack& d, bool* chan
       (rc = b.Xb.ensure(n)) || (rc = b.G.ensure(n)) || (rc = b.raw.ensure(n)) ||
       (rc = b.S.ensure((size_t)g.spec_elems())) ||
       (rc = b.partials.ensure(2 * (size_t)x_pass_blocks(g))) ||
-      (rc = b.lam.ensure(2)))
+      (rc = b.lam.ensure(4)))
     return rc;
   b.os.raw_otf = b.raw_otf.p;
   return 0;
@@ -1002,7 +1008,7 @@ static int batch_capture(Batch& b, int nIters, bool host) {
         break;
       ++launches;
     }
-    if ((e = cudaMemsetAsync(t.lam.p, 0, 2 * sizeof(float), s)) != cudaSuccess ||
+    if ((e = cudaMemsetAsync(t.lam.p, 0, 4 * sizeof(float), s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(t.raw.p, t.Xa.p, n * sizeof(float), cudaMemcpyDeviceToDevice, s)) !=
             cudaSuccess) {
       set_cuda_error("batch capture", e);

@@ -344,7 +344,7 @@ struct RatioRange {
 template <class PL, int NQ>
 __global__ void __launch_bounds__(PX<PL, NQ>::T, PX<PL, NQ>::kBlocks)
 k_px_ratio(PairGeom g, const float2* __restrict__ tw, float4* S, const float* __restrict__ raw,
-           float eps) {
+           const float* mean, float eps) {
   using P = PX<PL, NQ>;
   extern __shared__ __align__(16) float2 smem[];
   float2* stw = smem;
@@ -354,6 +354,7 @@ k_px_ratio(PairGeom g, const float2* __restrict__ tw, float4* S, const float* __
   prefetch_rows<NQ>(g, P::rows(smem, 0), raw, z, m0);  // written before the iterations
   cp_async_commit();
   grid_dep_wait();
+  const float2 off = dup2(mean ? -__ldcg(mean) : 0.f);
   spec_to_tile<PL, NQ, false>(g, sm, stw, S, z, m0, [] {});
   const int idx = threadIdx.x;
   const int q = idx / PL::KC, k = idx - q * PL::KC;
@@ -383,15 +384,18 @@ k_px_ratio(PairGeom g, const float2* __restrict__ tw, float4* S, const float* __
         x[r].im = make_float2(rl_ratio(x[r].im.x, d[r].im.x, eps), rl_ratio(x[r].im.y, d[r].im.y, eps));
       }
     }
-    // The ratio goes on as ratio - 1: it lies around 1, and what the second
-    // convolution does to the 1 is known exactly (the OTF at frequency 0, added
-    // back by the update pass), so that its transforms round the small
-    // deviation instead of values near 1.  That rounding was most of the RL
-    // loop's error: 16-19 iterations of 34 stacks, relative to 64 bits, 9-51e-7
-    // before and 5-14e-7 with the 1 taken out.
+    // The ratio goes on less a constant m: what the second convolution does to a
+    // constant is known (m times the OTF at frequency 0, added back by the update
+    // pass), and its transforms round in proportion to the root mean square of
+    // what they are given.  That is smallest, and never more than the ratio's own,
+    // with m the ratio's mean; the mean of the iteration before (0 in the first)
+    // is at hand, as frequency 0 of that spectrum in the z pass, and close to it.
+    // The ratio is about 1 where the image is above the background and about 0
+    // where it is empty, so m lies near 1 in crowded images and near 0 in dark
+    // ones; a fixed 1 took the error of images with nine tenths of zeros up 1.5
+    // to 4 times.
 #pragma unroll
-    for (int r = 0; r < PL::Q2; ++r)
-      x[r] = {add2(x[r].re, dup2(-1.f)), add2(x[r].im, dup2(-1.f))};
+    for (int r = 0; r < PL::Q2; ++r) x[r] = {add2(x[r].re, off), add2(x[r].im, off)};
     if (!(rq.v2 && rq.v3)) {
 #pragma unroll
       for (int r = 0; r < PL::Q2; ++r) {
@@ -420,11 +424,11 @@ __device__ __forceinline__ void acc_add2(float2& hi, float2& lo, float2 p) {
 }
 
 // Y == nullptr: the plain inverse transform, written to Xout; otherwise h0 is
-// the OTF at frequency 0 (see k_px_ratio).
+// the OTF at frequency 0 and mean what k_px_ratio took off the ratio.
 template <class PL, int NQ, int STAGED>
 __global__ void __launch_bounds__(PX<PL, NQ>::T, PX<PL, NQ>::blocks_upd(STAGED))
 k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y, float* Xout,
-            float* G, int dots, float4* partials, const float* h0) {
+            float* G, int dots, float4* partials, const float* h0, const float* mean) {
   using P = PX<PL, NQ>;
   extern __shared__ __align__(16) float2 smem[];
   __shared__ float4 red[32];
@@ -484,9 +488,9 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
   // 16 bytes an access where they are aligned.  X is read next
   // by the x forward pass (kept in L2), G only by the next iteration's update.
   float2 s1h = make_float2(0.f, 0.f), s1l = s1h, s2h = s1h, s2l = s1h;
-  const float2 one = dup2(Y ? __ldg(h0) : 0.f);
+  const float2 add = dup2(Y && mean ? __ldcg(mean) * __ldg(h0) : 0.f);
   auto update = [&](float2 cc, float2 y, float2 go, float2& xn, float2& gn) {
-    xn = relu2(mul2(add2(cc, one), y));
+    xn = relu2(mul2(add2(cc, add), y));
     gn = sub2(xn, y);
     if (dots) {
       acc_add2(s1h, s1l, mul2(gn, go));
@@ -599,15 +603,15 @@ static int px_fwd_go(const PairGeom& g, const float2* tw, const float* X, float*
 }
 
 template <class PL, int NQ>
-static int px_ratio_go(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps,
-                       cudaStream_t st) {
+static int px_ratio_go(const PairGeom& g, const float2* tw, float2* S, const float* raw,
+                       const float* mean, float eps, cudaStream_t st) {
   using P = PX<PL, NQ>;
   static_assert(P::kBlocks > 0, "an SM holds a block");
   auto kern = k_px_ratio<PL, NQ>;
   const size_t smem = P::smem(1);
   if (int rc = smem_optin(kern, smem)) return rc;
   CDX_CHECK(launch_pdl(kern, dim3(ceil_div(g.H / 2, NQ), g.nz), dim3(P::T), smem, st, g, tw,
-                       reinterpret_cast<float4*>(S), raw, eps));
+                       reinterpret_cast<float4*>(S), raw, mean, eps));
   CDX_LAUNCH_CHECK("k_px_ratio");
   return 0;
 }
@@ -635,10 +639,10 @@ static int px_update_go(const PairGeom& g, const float2* tw, const float2* S, co
   const size_t smem = P::smem(stage ? P::kStaged : 0);
   if (int rc = smem_optin(kern, smem)) return rc;
   float4* part = dots ? reinterpret_cast<float4*>(w->partials) : nullptr;
-  const float* h0 = w ? w->h0 : nullptr;
+  const float *h0 = w ? w->h0 : nullptr, *mean = w ? w->mean : nullptr;
   CDX_CHECK(launch_pdl(kern, grid, dim3(P::T), smem, st, g, tw,
                        reinterpret_cast<float4*>(const_cast<float2*>(S)), Y, Xout, G, dots, part,
-                       h0));
+                       h0, mean));
   CDX_LAUNCH_CHECK("k_px_update");
   if (dots) return launch_lambda(part, nblk, lam_next, eps, st);
   return 0;

@@ -25,6 +25,15 @@ struct PZ {
   static_assert(T % W == 0 && kBlocks > 0, "a thread copies one column, an SM holds a block");
 };
 
+// The mean of the ratio whose spectrum the z pass holds, for the next iteration
+// (k_px_ratio): what was taken off it plus what is left at frequency 0 (twice the
+// transform, as the paired passes have it).  The ratio lies within 10; a mean that
+// does not (NaN, when the image holds one) gives 0.
+__device__ __forceinline__ void store_ratio_mean(const OtfDev& otf, float freq0) {
+  const float m = __fmaf_rn(freq0, otf.inv2n, otf.mean ? __ldcg(otf.mean) : 0.f);
+  *otf.mean_next = fabsf(m) <= 10.f ? m : 0.f;
+}
+
 // MODE 0: radially averaged table (CONJ: its conjugate); 1: full 3D array in
 // the paired layout, conjugated when conj, or with fwd_only the forward
 // transform alone.
@@ -107,6 +116,8 @@ k_pz(PairGeom g, const float2* __restrict__ tw, float4* S, OtfDev otf, int conj,
 #pragma unroll
       for (int r = 0; r < Q2; ++r) x[r] = ldp(p + r * W);
       butterfly<Q2, KC, false, false>(x, stw, b);
+      if ((CONJ || MODE == 1) && otf.mean_next && b == 0 && kx == 0 && s == 0)
+        store_ratio_mean(otf, x[0].re.x);
       if (MODE == 1 && fwd_only) {
         if (in) {
 #pragma unroll

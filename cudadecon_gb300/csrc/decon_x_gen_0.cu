@@ -34,29 +34,29 @@ int pxgen_fwd_0(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
   }
 }
 
-int pxgen_ratio_0(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_0(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 128:
       *done = true;
-      return px_ratio_go<PPX128, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX128, 2>(g, tw, S, raw, mean, eps, st);
     case 243:
       *done = true;
-      return px_ratio_go<PPX243, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX243, 2>(g, tw, S, raw, mean, eps, st);
     case 392:
       *done = true;
-      return px_ratio_go<PPX392, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX392, 2>(g, tw, S, raw, mean, eps, st);
     case 600:
       *done = true;
-      return px_ratio_go<PPX600, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX600, 2>(g, tw, S, raw, mean, eps, st);
     case 875:
       *done = true;
-      return px_ratio_go<PPX875, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX875, 2>(g, tw, S, raw, mean, eps, st);
     case 1215:
       *done = true;
-      return px_ratio_go<PPX1215, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1215, 2>(g, tw, S, raw, mean, eps, st);
     case 1620:
       *done = true;
-      return px_ratio_go<PPX1620, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1620, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_1(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
   }
 }
 
-int pxgen_ratio_1(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_1(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 135:
       *done = true;
-      return px_ratio_go<PPX135, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX135, 2>(g, tw, S, raw, mean, eps, st);
     case 245:
       *done = true;
-      return px_ratio_go<PPX245, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX245, 2>(g, tw, S, raw, mean, eps, st);
     case 400:
       *done = true;
-      return px_ratio_go<PPX400, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX400, 2>(g, tw, S, raw, mean, eps, st);
     case 625:
       *done = true;
-      return px_ratio_go<PPX625, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX625, 2>(g, tw, S, raw, mean, eps, st);
     case 882:
       *done = true;
-      return px_ratio_go<PPX882, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX882, 2>(g, tw, S, raw, mean, eps, st);
     case 1225:
       *done = true;
-      return px_ratio_go<PPX1225, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1225, 2>(g, tw, S, raw, mean, eps, st);
     case 1680:
       *done = true;
-      return px_ratio_go<PPX1680, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1680, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_10(const PairGeom& g, const float2* tw, const float* X, float* Xm1
   }
 }
 
-int pxgen_ratio_10(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_10(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 180:
       *done = true;
-      return px_ratio_go<PPX180, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX180, 2>(g, tw, S, raw, mean, eps, st);
     case 315:
       *done = true;
-      return px_ratio_go<PPX315, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX315, 2>(g, tw, S, raw, mean, eps, st);
     case 490:
       *done = true;
-      return px_ratio_go<PPX490, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX490, 2>(g, tw, S, raw, mean, eps, st);
     case 729:
       *done = true;
-      return px_ratio_go<PPX729, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX729, 2>(g, tw, S, raw, mean, eps, st);
     case 1024:
       *done = true;
-      return px_ratio_go<PPX1024, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1024, 2>(g, tw, S, raw, mean, eps, st);
     case 1400:
       *done = true;
-      return px_ratio_go<PPX1400, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1400, 2>(g, tw, S, raw, mean, eps, st);
     case 1920:
       *done = true;
-      return px_ratio_go<PPX1920, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1920, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_11(const PairGeom& g, const float2* tw, const float* X, float* Xm1
   }
 }
 
-int pxgen_ratio_11(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_11(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 189:
       *done = true;
-      return px_ratio_go<PPX189, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX189, 2>(g, tw, S, raw, mean, eps, st);
     case 320:
       *done = true;
-      return px_ratio_go<PPX320, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX320, 2>(g, tw, S, raw, mean, eps, st);
     case 500:
       *done = true;
-      return px_ratio_go<PPX500, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX500, 2>(g, tw, S, raw, mean, eps, st);
     case 735:
       *done = true;
-      return px_ratio_go<PPX735, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX735, 2>(g, tw, S, raw, mean, eps, st);
     case 1029:
       *done = true;
-      return px_ratio_go<PPX1029, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1029, 2>(g, tw, S, raw, mean, eps, st);
     case 1440:
       *done = true;
-      return px_ratio_go<PPX1440, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1440, 2>(g, tw, S, raw, mean, eps, st);
     case 1944:
       *done = true;
-      return px_ratio_go<PPX1944, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1944, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_12(const PairGeom& g, const float2* tw, const float* X, float* Xm1
   }
 }
 
-int pxgen_ratio_12(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_12(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 192:
       *done = true;
-      return px_ratio_go<PPX192, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX192, 2>(g, tw, S, raw, mean, eps, st);
     case 324:
       *done = true;
-      return px_ratio_go<PPX324, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX324, 2>(g, tw, S, raw, mean, eps, st);
     case 504:
       *done = true;
-      return px_ratio_go<PPX504, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX504, 2>(g, tw, S, raw, mean, eps, st);
     case 750:
       *done = true;
-      return px_ratio_go<PPX750, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX750, 2>(g, tw, S, raw, mean, eps, st);
     case 1050:
       *done = true;
-      return px_ratio_go<PPX1050, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1050, 2>(g, tw, S, raw, mean, eps, st);
     case 1458:
       *done = true;
-      return px_ratio_go<PPX1458, 4>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1458, 4>(g, tw, S, raw, mean, eps, st);
     case 1960:
       *done = true;
-      return px_ratio_go<PPX1960, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1960, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_13(const PairGeom& g, const float2* tw, const float* X, float* Xm1
   }
 }
 
-int pxgen_ratio_13(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_13(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 196:
       *done = true;
-      return px_ratio_go<PPX196, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX196, 2>(g, tw, S, raw, mean, eps, st);
     case 336:
       *done = true;
-      return px_ratio_go<PPX336, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX336, 2>(g, tw, S, raw, mean, eps, st);
     case 512:
       *done = true;
-      return px_ratio_go<PPX512, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX512, 2>(g, tw, S, raw, mean, eps, st);
     case 756:
       *done = true;
-      return px_ratio_go<PPX756, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX756, 2>(g, tw, S, raw, mean, eps, st);
     case 1080:
       *done = true;
-      return px_ratio_go<PPX1080, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1080, 2>(g, tw, S, raw, mean, eps, st);
     case 1470:
       *done = true;
-      return px_ratio_go<PPX1470, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1470, 2>(g, tw, S, raw, mean, eps, st);
     case 2000:
       *done = true;
-      return px_ratio_go<PPX2000, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX2000, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_14(const PairGeom& g, const float2* tw, const float* X, float* Xm1
   }
 }
 
-int pxgen_ratio_14(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_14(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 200:
       *done = true;
-      return px_ratio_go<PPX200, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX200, 2>(g, tw, S, raw, mean, eps, st);
     case 343:
       *done = true;
-      return px_ratio_go<PPX343, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX343, 2>(g, tw, S, raw, mean, eps, st);
     case 525:
       *done = true;
-      return px_ratio_go<PPX525, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX525, 2>(g, tw, S, raw, mean, eps, st);
     case 768:
       *done = true;
-      return px_ratio_go<PPX768, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX768, 2>(g, tw, S, raw, mean, eps, st);
     case 1120:
       *done = true;
-      return px_ratio_go<PPX1120, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1120, 2>(g, tw, S, raw, mean, eps, st);
     case 1500:
       *done = true;
-      return px_ratio_go<PPX1500, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1500, 2>(g, tw, S, raw, mean, eps, st);
     case 2016:
       *done = true;
-      return px_ratio_go<PPX2016, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX2016, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_15(const PairGeom& g, const float2* tw, const float* X, float* Xm1
   }
 }
 
-int pxgen_ratio_15(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_15(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 210:
       *done = true;
-      return px_ratio_go<PPX210, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX210, 2>(g, tw, S, raw, mean, eps, st);
     case 350:
       *done = true;
-      return px_ratio_go<PPX350, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX350, 2>(g, tw, S, raw, mean, eps, st);
     case 540:
       *done = true;
-      return px_ratio_go<PPX540, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX540, 2>(g, tw, S, raw, mean, eps, st);
     case 784:
       *done = true;
-      return px_ratio_go<PPX784, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX784, 2>(g, tw, S, raw, mean, eps, st);
     case 1125:
       *done = true;
-      return px_ratio_go<PPX1125, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1125, 2>(g, tw, S, raw, mean, eps, st);
     case 1512:
       *done = true;
-      return px_ratio_go<PPX1512, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1512, 2>(g, tw, S, raw, mean, eps, st);
     case 2025:
       *done = true;
-      return px_ratio_go<PPX2025, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX2025, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_16(const PairGeom& g, const float2* tw, const float* X, float* Xm1
   }
 }
 
-int pxgen_ratio_16(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_16(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 216:
       *done = true;
-      return px_ratio_go<PPX216, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX216, 2>(g, tw, S, raw, mean, eps, st);
     case 360:
       *done = true;
-      return px_ratio_go<PPX360, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX360, 2>(g, tw, S, raw, mean, eps, st);
     case 560:
       *done = true;
-      return px_ratio_go<PPX560, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX560, 2>(g, tw, S, raw, mean, eps, st);
     case 800:
       *done = true;
-      return px_ratio_go<PPX800, 4>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX800, 4>(g, tw, S, raw, mean, eps, st);
     case 1134:
       *done = true;
-      return px_ratio_go<PPX1134, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1134, 2>(g, tw, S, raw, mean, eps, st);
     case 1536:
       *done = true;
-      return px_ratio_go<PPX1536, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1536, 2>(g, tw, S, raw, mean, eps, st);
     case 2048:
       *done = true;
-      return px_ratio_go<PPX2048, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX2048, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -31,26 +31,26 @@ int pxgen_fwd_17(const PairGeom& g, const float2* tw, const float* X, float* Xm1
   }
 }
 
-int pxgen_ratio_17(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_17(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 224:
       *done = true;
-      return px_ratio_go<PPX224, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX224, 2>(g, tw, S, raw, mean, eps, st);
     case 375:
       *done = true;
-      return px_ratio_go<PPX375, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX375, 2>(g, tw, S, raw, mean, eps, st);
     case 567:
       *done = true;
-      return px_ratio_go<PPX567, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX567, 2>(g, tw, S, raw, mean, eps, st);
     case 810:
       *done = true;
-      return px_ratio_go<PPX810, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX810, 2>(g, tw, S, raw, mean, eps, st);
     case 1152:
       *done = true;
-      return px_ratio_go<PPX1152, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1152, 2>(g, tw, S, raw, mean, eps, st);
     case 1568:
       *done = true;
-      return px_ratio_go<PPX1568, 4>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1568, 4>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

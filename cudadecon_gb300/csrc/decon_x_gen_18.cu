@@ -31,26 +31,26 @@ int pxgen_fwd_18(const PairGeom& g, const float2* tw, const float* X, float* Xm1
   }
 }
 
-int pxgen_ratio_18(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_18(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 225:
       *done = true;
-      return px_ratio_go<PPX225, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX225, 2>(g, tw, S, raw, mean, eps, st);
     case 378:
       *done = true;
-      return px_ratio_go<PPX378, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX378, 2>(g, tw, S, raw, mean, eps, st);
     case 576:
       *done = true;
-      return px_ratio_go<PPX576, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX576, 2>(g, tw, S, raw, mean, eps, st);
     case 840:
       *done = true;
-      return px_ratio_go<PPX840, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX840, 2>(g, tw, S, raw, mean, eps, st);
     case 1176:
       *done = true;
-      return px_ratio_go<PPX1176, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1176, 2>(g, tw, S, raw, mean, eps, st);
     case 1575:
       *done = true;
-      return px_ratio_go<PPX1575, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1575, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -31,26 +31,26 @@ int pxgen_fwd_19(const PairGeom& g, const float2* tw, const float* X, float* Xm1
   }
 }
 
-int pxgen_ratio_19(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_19(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 240:
       *done = true;
-      return px_ratio_go<PPX240, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX240, 2>(g, tw, S, raw, mean, eps, st);
     case 384:
       *done = true;
-      return px_ratio_go<PPX384, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX384, 2>(g, tw, S, raw, mean, eps, st);
     case 588:
       *done = true;
-      return px_ratio_go<PPX588, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX588, 2>(g, tw, S, raw, mean, eps, st);
     case 864:
       *done = true;
-      return px_ratio_go<PPX864, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX864, 2>(g, tw, S, raw, mean, eps, st);
     case 1200:
       *done = true;
-      return px_ratio_go<PPX1200, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1200, 2>(g, tw, S, raw, mean, eps, st);
     case 1600:
       *done = true;
-      return px_ratio_go<PPX1600, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1600, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

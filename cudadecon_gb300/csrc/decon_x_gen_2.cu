@@ -34,29 +34,29 @@ int pxgen_fwd_2(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
   }
 }
 
-int pxgen_ratio_2(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_2(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 140:
       *done = true;
-      return px_ratio_go<PPX140, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX140, 2>(g, tw, S, raw, mean, eps, st);
     case 250:
       *done = true;
-      return px_ratio_go<PPX250, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX250, 2>(g, tw, S, raw, mean, eps, st);
     case 405:
       *done = true;
-      return px_ratio_go<PPX405, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX405, 2>(g, tw, S, raw, mean, eps, st);
     case 630:
       *done = true;
-      return px_ratio_go<PPX630, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX630, 2>(g, tw, S, raw, mean, eps, st);
     case 896:
       *done = true;
-      return px_ratio_go<PPX896, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX896, 2>(g, tw, S, raw, mean, eps, st);
     case 1250:
       *done = true;
-      return px_ratio_go<PPX1250, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1250, 2>(g, tw, S, raw, mean, eps, st);
     case 1701:
       *done = true;
-      return px_ratio_go<PPX1701, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1701, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

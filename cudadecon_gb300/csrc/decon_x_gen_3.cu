@@ -34,29 +34,29 @@ int pxgen_fwd_3(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
   }
 }
 
-int pxgen_ratio_3(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_3(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 144:
       *done = true;
-      return px_ratio_go<PPX144, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX144, 2>(g, tw, S, raw, mean, eps, st);
     case 252:
       *done = true;
-      return px_ratio_go<PPX252, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX252, 2>(g, tw, S, raw, mean, eps, st);
     case 420:
       *done = true;
-      return px_ratio_go<PPX420, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX420, 2>(g, tw, S, raw, mean, eps, st);
     case 640:
       *done = true;
-      return px_ratio_go<PPX640, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX640, 2>(g, tw, S, raw, mean, eps, st);
     case 900:
       *done = true;
-      return px_ratio_go<PPX900, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX900, 2>(g, tw, S, raw, mean, eps, st);
     case 1260:
       *done = true;
-      return px_ratio_go<PPX1260, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1260, 2>(g, tw, S, raw, mean, eps, st);
     case 1728:
       *done = true;
-      return px_ratio_go<PPX1728, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1728, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_4(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
   }
 }
 
-int pxgen_ratio_4(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_4(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 147:
       *done = true;
-      return px_ratio_go<PPX147, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX147, 2>(g, tw, S, raw, mean, eps, st);
     case 256:
       *done = true;
-      return px_ratio_go<PPX256, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX256, 2>(g, tw, S, raw, mean, eps, st);
     case 432:
       *done = true;
-      return px_ratio_go<PPX432, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX432, 2>(g, tw, S, raw, mean, eps, st);
     case 648:
       *done = true;
-      return px_ratio_go<PPX648, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX648, 2>(g, tw, S, raw, mean, eps, st);
     case 945:
       *done = true;
-      return px_ratio_go<PPX945, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX945, 2>(g, tw, S, raw, mean, eps, st);
     case 1280:
       *done = true;
-      return px_ratio_go<PPX1280, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1280, 2>(g, tw, S, raw, mean, eps, st);
     case 1750:
       *done = true;
-      return px_ratio_go<PPX1750, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1750, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_5(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
   }
 }
 
-int pxgen_ratio_5(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_5(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 150:
       *done = true;
-      return px_ratio_go<PPX150, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX150, 2>(g, tw, S, raw, mean, eps, st);
     case 270:
       *done = true;
-      return px_ratio_go<PPX270, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX270, 2>(g, tw, S, raw, mean, eps, st);
     case 441:
       *done = true;
-      return px_ratio_go<PPX441, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX441, 2>(g, tw, S, raw, mean, eps, st);
     case 672:
       *done = true;
-      return px_ratio_go<PPX672, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX672, 2>(g, tw, S, raw, mean, eps, st);
     case 960:
       *done = true;
-      return px_ratio_go<PPX960, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX960, 2>(g, tw, S, raw, mean, eps, st);
     case 1296:
       *done = true;
-      return px_ratio_go<PPX1296, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1296, 2>(g, tw, S, raw, mean, eps, st);
     case 1764:
       *done = true;
-      return px_ratio_go<PPX1764, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1764, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_6(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
   }
 }
 
-int pxgen_ratio_6(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_6(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 160:
       *done = true;
-      return px_ratio_go<PPX160, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX160, 2>(g, tw, S, raw, mean, eps, st);
     case 280:
       *done = true;
-      return px_ratio_go<PPX280, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX280, 2>(g, tw, S, raw, mean, eps, st);
     case 448:
       *done = true;
-      return px_ratio_go<PPX448, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX448, 2>(g, tw, S, raw, mean, eps, st);
     case 675:
       *done = true;
-      return px_ratio_go<PPX675, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX675, 2>(g, tw, S, raw, mean, eps, st);
     case 972:
       *done = true;
-      return px_ratio_go<PPX972, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX972, 2>(g, tw, S, raw, mean, eps, st);
     case 1323:
       *done = true;
-      return px_ratio_go<PPX1323, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1323, 2>(g, tw, S, raw, mean, eps, st);
     case 1792:
       *done = true;
-      return px_ratio_go<PPX1792, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1792, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_7(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
   }
 }
 
-int pxgen_ratio_7(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_7(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 162:
       *done = true;
-      return px_ratio_go<PPX162, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX162, 2>(g, tw, S, raw, mean, eps, st);
     case 288:
       *done = true;
-      return px_ratio_go<PPX288, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX288, 2>(g, tw, S, raw, mean, eps, st);
     case 450:
       *done = true;
-      return px_ratio_go<PPX450, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX450, 2>(g, tw, S, raw, mean, eps, st);
     case 686:
       *done = true;
-      return px_ratio_go<PPX686, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX686, 2>(g, tw, S, raw, mean, eps, st);
     case 980:
       *done = true;
-      return px_ratio_go<PPX980, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX980, 2>(g, tw, S, raw, mean, eps, st);
     case 1344:
       *done = true;
-      return px_ratio_go<PPX1344, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1344, 2>(g, tw, S, raw, mean, eps, st);
     case 1800:
       *done = true;
-      return px_ratio_go<PPX1800, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1800, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

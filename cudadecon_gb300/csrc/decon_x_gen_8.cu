@@ -34,29 +34,29 @@ int pxgen_fwd_8(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
   }
 }
 
-int pxgen_ratio_8(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_8(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 168:
       *done = true;
-      return px_ratio_go<PPX168, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX168, 2>(g, tw, S, raw, mean, eps, st);
     case 294:
       *done = true;
-      return px_ratio_go<PPX294, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX294, 2>(g, tw, S, raw, mean, eps, st);
     case 480:
       *done = true;
-      return px_ratio_go<PPX480, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX480, 2>(g, tw, S, raw, mean, eps, st);
     case 700:
       *done = true;
-      return px_ratio_go<PPX700, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX700, 2>(g, tw, S, raw, mean, eps, st);
     case 1000:
       *done = true;
-      return px_ratio_go<PPX1000, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1000, 2>(g, tw, S, raw, mean, eps, st);
     case 1350:
       *done = true;
-      return px_ratio_go<PPX1350, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1350, 2>(g, tw, S, raw, mean, eps, st);
     case 1875:
       *done = true;
-      return px_ratio_go<PPX1875, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1875, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -34,29 +34,29 @@ int pxgen_fwd_9(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
   }
 }
 
-int pxgen_ratio_9(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+int pxgen_ratio_9(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   switch (g.nx) {
     case 175:
       *done = true;
-      return px_ratio_go<PPX175, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX175, 2>(g, tw, S, raw, mean, eps, st);
     case 300:
       *done = true;
-      return px_ratio_go<PPX300, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX300, 2>(g, tw, S, raw, mean, eps, st);
     case 486:
       *done = true;
-      return px_ratio_go<PPX486, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX486, 2>(g, tw, S, raw, mean, eps, st);
     case 720:
       *done = true;
-      return px_ratio_go<PPX720, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX720, 2>(g, tw, S, raw, mean, eps, st);
     case 1008:
       *done = true;
-      return px_ratio_go<PPX1008, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1008, 2>(g, tw, S, raw, mean, eps, st);
     case 1372:
       *done = true;
-      return px_ratio_go<PPX1372, 4>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1372, 4>(g, tw, S, raw, mean, eps, st);
     case 1890:
       *done = true;
-      return px_ratio_go<PPX1890, 2>(g, tw, S, raw, eps, st);
+      return px_ratio_go<PPX1890, 2>(g, tw, S, raw, mean, eps, st);
     default:
       return 0;
   }

@@ -6,10 +6,10 @@
 namespace cdx {
 
 int launch_x_inv_ratio_fwd(const Geom& g, const FftLen& fx, float2* S, const float* raw,
-                           float eps, cudaStream_t st) {
+                           const float* mean, float eps, cudaStream_t st) {
   if (g.pair) {
     bool done = false;
-    const int rc = pxgen_ratio(pair_geom(g), fx.d_pair, S, raw, eps, st, &done);
+    const int rc = pxgen_ratio(pair_geom(g), fx.d_pair, S, raw, mean, eps, st, &done);
     if (done || rc) return rc;
   }
   if (fx.has_tc && dft_form() == 1)

@@ -27,26 +27,26 @@ int pxgen_fwd_16(const PairGeom& g, const float2* tw, const float* X, float* Xm1
 int pxgen_fwd_17(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
 int pxgen_fwd_18(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
 int pxgen_fwd_19(const PairGeom& g, const float2* tw, const float* X, float* Xm1, const float* lam, int predict, float bg, float2* S, cudaStream_t st, bool* done);
-int pxgen_ratio_0(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_1(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_2(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_3(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_4(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_5(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_6(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_7(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_8(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_9(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_10(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_11(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_12(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_13(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_14(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_15(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_16(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_17(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_18(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
-int pxgen_ratio_19(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_0(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_1(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_2(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_3(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_4(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_5(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_6(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_7(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_8(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_9(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_10(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_11(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_12(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_13(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_14(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_15(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_16(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_17(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_18(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
+int pxgen_ratio_19(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done);
 int pxgen_update_0(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done);
 int pxgen_update_1(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done);
 int pxgen_update_2(const PairGeom& g, const float2* tw, const float2* S, const float* Y, float* Xout, float* G, int dots, RLWork* w, float* lam_next, float eps, cudaStream_t st, bool* done);
@@ -110,29 +110,29 @@ inline int pxgen_fwd(const PairGeom& g, const float2* tw, const float* X, float*
   return 0;
 }
 
-inline int pxgen_ratio(const PairGeom& g, const float2* tw, float2* S, const float* raw, float eps, cudaStream_t st, bool* done) {
+inline int pxgen_ratio(const PairGeom& g, const float2* tw, float2* S, const float* raw, const float* mean, float eps, cudaStream_t st, bool* done) {
   int rc = 0;
   *done = false;
-  if ((rc = pxgen_ratio_0(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_1(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_2(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_3(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_4(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_5(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_6(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_7(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_8(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_9(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_10(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_11(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_12(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_13(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_14(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_15(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_16(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_17(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_18(g, tw, S, raw, eps, st, done)) || *done) return rc;
-  if ((rc = pxgen_ratio_19(g, tw, S, raw, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_0(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_1(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_2(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_3(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_4(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_5(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_6(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_7(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_8(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_9(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_10(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_11(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_12(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_13(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_14(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_15(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_16(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_17(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_18(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
+  if ((rc = pxgen_ratio_19(g, tw, S, raw, mean, eps, st, done)) || *done) return rc;
   return 0;
 }
 

@@ -472,7 +472,7 @@ def pair_units() -> dict:
             "pxgen_fwd": ("const PairGeom& g, const float2* tw, const float* X, float* Xm1, "
                           "const float* lam, int predict, float bg, float2* S", "px_fwd_go", X_UNITS),
             "pxgen_ratio": ("const PairGeom& g, const float2* tw, float2* S, const float* raw, "
-                            "float eps", "px_ratio_go", X_UNITS),
+                            "const float* mean, float eps", "px_ratio_go", X_UNITS),
             "pxgen_update": ("const PairGeom& g, const float2* tw, const float2* S, const float* Y, "
                              "float* Xout, float* G, int dots, RLWork* w, float* lam_next, "
                              "float eps", "px_update_go", X_UNITS),
