@@ -373,6 +373,11 @@ static int ensure_plan(Session& s, int gx, int gy, int gz) {
   return 0;
 }
 
+// Floats of LoopBufs::lam: two lambda slots, the means taken off the first, the
+// second and the later ratios, and those means convolved.  All 0 at the start of a
+// loop.
+constexpr int kLoopScalars = 8;
+
 static int ensure_grid_buffers(Session& s, const Geom& g) {
   const size_t n = (size_t)g.nvox();
   int rc;
@@ -380,8 +385,8 @@ static int ensure_grid_buffers(Session& s, const Geom& g) {
       (rc = s.raw.ensure(n)) || (rc = s.S.ensure((size_t)g.spec_elems())))
     return rc;
   const int nblk = x_pass_blocks(g);
-  if ((rc = s.partials.ensure(2 * (size_t)nblk)) || (rc = s.lam.ensure(4))) return rc;
-  CDX_CHECK(cudaMemsetAsync(s.lam.p, 0, 4 * sizeof(float), s.stream));
+  if ((rc = s.partials.ensure(2 * (size_t)nblk)) || (rc = s.lam.ensure(kLoopScalars))) return rc;
+  CDX_CHECK(cudaMemsetAsync(s.lam.p, 0, kLoopScalars * sizeof(float), s.stream));
   return 0;
 }
 
@@ -390,8 +395,7 @@ static int ensure_grid_buffers(Session& s, const Geom& g) {
 // the grid of s.plan, starting from X0 in s.Xa with raw in s.raw.  Returns
 // the buffer that holds the final estimate.
 // Device buffers of one RL loop: estimates (X0 in Xa), raw, G, spectrum,
-// dot-product partials (16 bytes per x-pass block), two lambda slots and, behind
-// them, two for the mean of the ratio.
+// dot-product partials (16 bytes per x-pass block) and kLoopScalars floats.
 struct LoopBufs {
   float* Xa;
   float* Xb;
@@ -412,8 +416,7 @@ static int rl_loop(const GridPlan& p, const LoopBufs& b, int nIter, cudaStream_t
   w.partials = b.partials;
   w.lam = b.lam;
   w.max_blocks = b.max_blocks;
-  w.h0 = p.otf.h0;
-  OtfDev conj = p.otf;  // second convolution: keeps the ratio's mean as it passes
+  OtfDev conj = p.otf;  // second convolution: stores the ratio's mean
   conj.inv2n = (float)(0.5 / (double)g.nvox());
   const float eps = 1.1920928955078125e-07f;  // std::numeric_limits<float>::epsilon()
   float* X = b.Xa;
@@ -438,10 +441,12 @@ static int rl_loop(const GridPlan& p, const LoopBufs& b, int nIter, cudaStream_t
     mark();
     if ((rc = launch_y_pass(g, p.fy, b.S, true, st))) return rc;
     mark();
-    // the mean of the last iteration's ratio is taken off this one's
-    w.mean = conj.mean = k > 0 ? b.lam + 2 + (k & 1) : nullptr;
-    conj.mean_next = b.lam + 2 + ((k + 1) & 1);
-    if ((rc = launch_x_inv_ratio_fwd(g, p.fx, b.S, b.raw, w.mean, eps, st))) return rc;
+    // nothing is taken off the first ratio, the first ratio's mean off the second,
+    // the second's off all that follow (measured anew each time the error is the same)
+    conj.mean = b.lam + 2 + std::min(k, 2);
+    conj.mean_next = k < 2 ? b.lam + 3 + k : nullptr;
+    w.add = conj.mean + 3;
+    if ((rc = launch_x_inv_ratio_fwd(g, p.fx, b.S, b.raw, conj.mean, eps, st))) return rc;
     mark();
     if ((rc = launch_y_pass(g, p.fy, b.S, false, st))) return rc;
     mark();
@@ -461,6 +466,7 @@ static int rl_loop(const GridPlan& p, const LoopBufs& b, int nIter, cudaStream_t
                                 st));
     if (prof && g_prof.used >= 10 * 64) prof_collect();
     *launches += k >= 1 ? 10 : 9;  // the update pass adds the lambda kernel
+    if (g.pair && k < 2 && (p.otf.mode == 1 || !p.fz.d_pair)) ++*launches;  // k_ratio_mean
     float* t = X;
     X = Xm1;
     Xm1 = t;
@@ -921,7 +927,7 @@ static int batch_setup_stack(BatchStack& b, const cdx_batch_stack& d, bool* chan
       (rc = b.Xb.ensure(n)) || (rc = b.G.ensure(n)) || (rc = b.raw.ensure(n)) ||
       (rc = b.S.ensure((size_t)g.spec_elems())) ||
       (rc = b.partials.ensure(2 * (size_t)x_pass_blocks(g))) ||
-      (rc = b.lam.ensure(4)))
+      (rc = b.lam.ensure(kLoopScalars)))
     return rc;
   b.os.raw_otf = b.raw_otf.p;
   return 0;
@@ -1008,7 +1014,7 @@ static int batch_capture(Batch& b, int nIters, bool host) {
         break;
       ++launches;
     }
-    if ((e = cudaMemsetAsync(t.lam.p, 0, 4 * sizeof(float), s)) != cudaSuccess ||
+    if ((e = cudaMemsetAsync(t.lam.p, 0, kLoopScalars * sizeof(float), s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(t.raw.p, t.Xa.p, n * sizeof(float), cudaMemcpyDeviceToDevice, s)) !=
             cudaSuccess) {
       set_cuda_error("batch capture", e);

@@ -354,8 +354,8 @@ k_px_ratio(PairGeom g, const float2* __restrict__ tw, float4* S, const float* __
   prefetch_rows<NQ>(g, P::rows(smem, 0), raw, z, m0);  // written before the iterations
   cp_async_commit();
   grid_dep_wait();
-  const float2 off = dup2(mean ? -__ldcg(mean) : 0.f);
-  spec_to_tile<PL, NQ, false>(g, sm, stw, S, z, m0, [] {});
+  float off = 0.f;
+  spec_to_tile<PL, NQ, false>(g, sm, stw, S, z, m0, [&] { off = -__ldg(mean); });
   const int idx = threadIdx.x;
   const int q = idx / PL::KC, k = idx - q * PL::KC;
   C2 x[PL::Q2];
@@ -388,14 +388,14 @@ k_px_ratio(PairGeom g, const float2* __restrict__ tw, float4* S, const float* __
     // constant is known (m times the OTF at frequency 0, added back by the update
     // pass), and its transforms round in proportion to the root mean square of
     // what they are given.  That is smallest, and never more than the ratio's own,
-    // with m the ratio's mean; the mean of the iteration before (0 in the first)
-    // is at hand, as frequency 0 of that spectrum in the z pass, and close to it.
+    // with m the ratio's mean.  The mean of an earlier iteration's ratio is close to
+    // it and at hand in the z pass, as frequency 0 of that spectrum (rl_loop).
     // The ratio is about 1 where the image is above the background and about 0
     // where it is empty, so m lies near 1 in crowded images and near 0 in dark
     // ones; a fixed 1 took the error of images with nine tenths of zeros up 1.5
     // to 4 times.
 #pragma unroll
-    for (int r = 0; r < PL::Q2; ++r) x[r] = {add2(x[r].re, off), add2(x[r].im, off)};
+    for (int r = 0; r < PL::Q2; ++r) x[r] = {add2(x[r].re, dup2(off)), add2(x[r].im, dup2(off))};
     if (!(rq.v2 && rq.v3)) {
 #pragma unroll
       for (int r = 0; r < PL::Q2; ++r) {
@@ -423,12 +423,12 @@ __device__ __forceinline__ void acc_add2(float2& hi, float2& lo, float2 p) {
   lo = add2(lo, err);
 }
 
-// Y == nullptr: the plain inverse transform, written to Xout; otherwise h0 is
-// the OTF at frequency 0 and mean what k_px_ratio took off the ratio.
+// Y == nullptr: the plain inverse transform, written to Xout; otherwise *addp is
+// what the convolution made of the constant that k_px_ratio took off.
 template <class PL, int NQ, int STAGED>
 __global__ void __launch_bounds__(PX<PL, NQ>::T, PX<PL, NQ>::blocks_upd(STAGED))
 k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y, float* Xout,
-            float* G, int dots, float4* partials, const float* h0, const float* mean) {
+            float* G, int dots, float4* partials, const float* addp) {
   using P = PX<PL, NQ>;
   extern __shared__ __align__(16) float2 smem[];
   __shared__ float4 red[32];
@@ -488,7 +488,7 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
   // 16 bytes an access where they are aligned.  X is read next
   // by the x forward pass (kept in L2), G only by the next iteration's update.
   float2 s1h = make_float2(0.f, 0.f), s1l = s1h, s2h = s1h, s2l = s1h;
-  const float2 add = dup2(Y && mean ? __ldcg(mean) * __ldg(h0) : 0.f);
+  const float2 add = dup2(Y ? __ldg(addp) : 0.f);
   auto update = [&](float2 cc, float2 y, float2 go, float2& xn, float2& gn) {
     xn = relu2(mul2(add2(cc, add), y));
     gn = sub2(xn, y);
@@ -639,10 +639,10 @@ static int px_update_go(const PairGeom& g, const float2* tw, const float2* S, co
   const size_t smem = P::smem(stage ? P::kStaged : 0);
   if (int rc = smem_optin(kern, smem)) return rc;
   float4* part = dots ? reinterpret_cast<float4*>(w->partials) : nullptr;
-  const float *h0 = w ? w->h0 : nullptr, *mean = w ? w->mean : nullptr;
+  const float* add = w ? w->add : nullptr;
   CDX_CHECK(launch_pdl(kern, grid, dim3(P::T), smem, st, g, tw,
                        reinterpret_cast<float4*>(const_cast<float2*>(S)), Y, Xout, G, dots, part,
-                       h0, mean));
+                       add));
   CDX_LAUNCH_CHECK("k_px_update");
   if (dots) return launch_lambda(part, nblk, lam_next, eps, st);
   return 0;

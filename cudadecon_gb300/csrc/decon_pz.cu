@@ -30,14 +30,12 @@ struct PairOtfStore {
   static constexpr bool kSmem = true;
   static constexpr bool kGroup = false;
   SmemIO io;
-  const OtfDev* mean;  // the tile with frequency 0 when it is to store the ratio's mean
   const float4* tz;
   const float* full;  // mode 1: float 0 of the tile's first slot at z = 0
   const int* cir;
   const float* car;
   int nr, rowf, nv, mode, conj;
   __device__ __forceinline__ void st(int v, int e, float2 x) const {
-    if (mean && v == 0 && e == 0) store_ratio_mean(*mean, x.x);
     float2 o = make_float2(0.f, 0.f);
     if (mode == 1) {
       if (v < nv) {
@@ -85,14 +83,26 @@ k_pz_gen(PairGeom g, FftDev fz, float4* S, OtfDev otf, int conj, int fwd_only, i
     return;
   }
   const float* full = otf.mode == 1 ? reinterpret_cast<const float*>(otf.full) + at : nullptr;
-  const bool first = blockIdx.x == 0 && blockIdx.y == 0;
-  const PairOtfStore ost{io, first && otf.mean_next ? &otf : nullptr, otf.tz, full, cir, car, otf.nr, 4 * g.zstep, nv, otf.mode, conj};
+  const PairOtfStore ost{io, otf.tz, full, cir, car, otf.nr, 4 * g.zstep, nv, otf.mode, conj};
   GenericRunner::run<false>(fz, W, invW, true, stw, io, gio, ost);
   GenericRunner::run<true>(fz, W, invW, true, stw, io, io, gio);
 }
 
+// The ratio's mean where the z kernels do not store it themselves: depths without a
+// plan and 3D OTFs.
+__global__ void __launch_bounds__(32) k_ratio_mean(PairGeom g, const float4* S, OtfDev otf) {
+  grid_dep_wait();
+  grid_dep_launch();
+  store_ratio_mean(g, S, otf);
+}
+
 int launch_pz(const PairGeom& g, const FftLen& fz, float2* S, const OtfDev& otf, bool conj,
               cudaStream_t st, bool fwd_only) {
+  if (otf.mean_next && (otf.mode == 1 || !fz.d_pair)) {
+    CDX_CHECK(launch_pdl(k_ratio_mean, dim3(1), dim3(32), 0, st, g,
+                         reinterpret_cast<const float4*>(S), otf));
+    CDX_LAUNCH_CHECK("k_ratio_mean");
+  }
   if (fz.d_pair) {
     bool done = false;
     const int rc = pzgen(g, fz.d_pair, S, otf, conj, st, fwd_only, &done);

@@ -25,13 +25,26 @@ struct PZ {
   static_assert(T % W == 0 && kBlocks > 0, "a thread copies one column, an SM holds a block");
 };
 
-// The mean of the ratio whose spectrum the z pass holds, for the next iteration
-// (k_px_ratio): what was taken off it plus what is left at frequency 0 (twice the
-// transform, as the paired passes have it).  The ratio lies within 10; a mean that
-// does not (NaN, when the image holds one) gives 0.
-__device__ __forceinline__ void store_ratio_mean(const OtfDev& otf, float freq0) {
-  const float m = __fmaf_rn(freq0, otf.inv2n, otf.mean ? __ldcg(otf.mean) : 0.f);
-  *otf.mean_next = fabsf(m) <= 10.f ? m : 0.f;
+// The mean of the ratio whose spectrum the z pass is given, for the next iteration
+// (k_px_ratio): what was taken off it plus what is left at frequency 0, the sum of
+// column (0, 0) over z (twice the transform, as the paired passes have it).  The
+// first warp of the block that has that column calls this before it is overwritten.
+// The ratio lies within 10; a mean that does not (NaN, when the image holds one)
+// gives 0.  Kernels of their own have it (MEAN), for two passes of a loop: in the
+// others, never reached, it cost 64 x 256 x 384 0.9% of an iteration.
+__device__ __forceinline__ void store_ratio_mean(const PairGeom& g, const float4* S,
+                                                 const OtfDev& otf) {
+  const float before = __ldcg(otf.mean), h0 = __ldg(otf.h0);
+  float sum = 0.f;
+#pragma unroll 4
+  for (int z = threadIdx.x; z < g.nz; z += 32)
+    sum += *reinterpret_cast<const float*>(S + (long long)z * g.zstep);
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if (threadIdx.x) return;
+  float m = __fmaf_rn(sum, otf.inv2n, before);
+  m = fabsf(m) <= 10.f ? m : 0.f;
+  otf.mean_next[0] = m;
+  otf.mean_next[3] = m * h0;
 }
 
 // MODE 0: radially averaged table (CONJ: its conjugate); 1: full 3D array in
@@ -42,7 +55,7 @@ __device__ __forceinline__ void store_ratio_mean(const OtfDev& otf, float freq0)
 // are on their way into the other half of its tile memory, so the latency of
 // global memory, which a block that loads, transforms and stores one tile
 // waits out (a third of its time), is hidden.
-template <class PL, int W, int MODE, bool CONJ>
+template <class PL, int W, int MODE, bool CONJ, bool MEAN>
 __global__ void __launch_bounds__(PZ<PL, W>::T, PZ<PL, W>::kBlocks)
 k_pz(PairGeom g, const float2* __restrict__ tw, float4* S, OtfDev otf, int conj, int fwd_only,
      int ntiles) {
@@ -74,6 +87,7 @@ k_pz(PairGeom g, const float2* __restrict__ tw, float4* S, OtfDev otf, int conj,
   int t = blockIdx.x;
   grid_dep_wait();
   if (t < ntiles) copy(t, bufs);
+  if (MEAN && blockIdx.x == 0 && threadIdx.x < 32) store_ratio_mean(g, S, otf);
   for (int half = 0; t < ntiles; t += gridDim.x, half ^= 1) {
     float4* tc = bufs + half * P::kTile + c;
     int kx, s;
@@ -116,8 +130,6 @@ k_pz(PairGeom g, const float2* __restrict__ tw, float4* S, OtfDev otf, int conj,
 #pragma unroll
       for (int r = 0; r < Q2; ++r) x[r] = ldp(p + r * W);
       butterfly<Q2, KC, false, false>(x, stw, b);
-      if ((CONJ || MODE == 1) && otf.mean_next && b == 0 && kx == 0 && s == 0)
-        store_ratio_mean(otf, x[0].re.x);
       if (MODE == 1 && fwd_only) {
         if (in) {
 #pragma unroll
@@ -171,11 +183,11 @@ k_pz(PairGeom g, const float2* __restrict__ tw, float4* S, OtfDev otf, int conj,
 }
 
 // ---------------------------------------------------------------- launches
-template <class PL, int W, int MODE, bool CONJ>
+template <class PL, int W, int MODE, bool CONJ, bool MEAN = false>
 static int pz_go(const PairGeom& g, const float2* tw, float2* S, const OtfDev& otf,
                  bool conj, cudaStream_t st, bool fwd_only) {
   using P = PZ<PL, W>;
-  auto kern = k_pz<PL, W, MODE, CONJ>;
+  auto kern = k_pz<PL, W, MODE, CONJ, MEAN>;
   if (int rc = smem_optin(kern, P::kSmem)) return rc;
   const int ntiles = ceil_div(4 * g.nxh, W) * ceil_div(g.slots, 4);
   const int grid = std::min(ntiles, P::kBlocks * sm_count());
@@ -189,6 +201,7 @@ template <class PL, int W>
 static int pz_mode(const PairGeom& g, const float2* tw, float2* S, const OtfDev& otf, bool conj,
                    cudaStream_t st, bool fwd_only) {
   if (fwd_only || otf.mode == 1) return pz_go<PL, W, 1, false>(g, tw, S, otf, conj, st, fwd_only);
+  if (otf.mean_next) return pz_go<PL, W, 0, true, true>(g, tw, S, otf, conj, st, false);
   return conj ? pz_go<PL, W, 0, true>(g, tw, S, otf, conj, st, false)
               : pz_go<PL, W, 0, false>(g, tw, S, otf, conj, st, false);
 }

@@ -380,7 +380,6 @@ template <bool INV, bool SYNC_MID, bool SYNC_END, class Ld, class St>
 __device__ __forceinline__ void stage_any(const StageDev& sd, int V, float invV, bool vfast,
                                           const float2* stw, const Ld& ld, const St& st) {
   switch (sd.R) {
-    case 1: stage_io<1, INV, SYNC_MID, SYNC_END>(sd, V, invV, vfast, stw, ld, st); break;
     case 2: stage_io<2, INV, SYNC_MID, SYNC_END>(sd, V, invV, vfast, stw, ld, st); break;
     case 3: stage_io<3, INV, SYNC_MID, SYNC_END>(sd, V, invV, vfast, stw, ld, st); break;
     case 4: stage_io<4, INV, SYNC_MID, SYNC_END>(sd, V, invV, vfast, stw, ld, st); break;
@@ -415,6 +414,10 @@ __device__ __forceinline__ void fft_run(const FftDev& f, int V, float invV, bool
                                         const float2* stw, const SmemIO& io, const Ld0& ld0,
                                         const StL& stL) {
   const int ns = f.nst;
+  if (f.L == 1) {
+    stage_io<1, INV, true, StL::kSmem>(f.st[0], V, invV, vfast, stw, ld0, stL);
+    return;
+  }
   if (ns == 1) {
     // a single stage may read and write the same rows (in place in global
     // memory too), so its reads and writes are always separated

@@ -51,8 +51,8 @@ struct OtfDev {
   const float2* full; // mode 1: spectrum-layout OTF, scaled by 1/N
   const float* h0;    // the raw OTF's value at frequency 0 (real part)
   // paired passes, second convolution of an iteration: the mean that was taken off
-  // the ratio (nullptr: 0) and where the ratio's own mean goes, from frequency 0
-  // of its spectrum times inv2n (0.5 / voxels)
+  // the ratio, and where the ratio's own mean goes if it is wanted (inv2n: 0.5 /
+  // voxels); three floats further, that mean times h0
   const float* mean;
   float* mean_next;
   float inv2n;
@@ -124,10 +124,9 @@ struct RLWork {
   double* partials = nullptr;   // 2 * max_blocks (16 bytes per x-pass block)
   float* lam = nullptr;         // two slots: lambda used by iteration k is lam[k & 1]
   int max_blocks = 0;
-  // paired passes: OTF value at frequency 0 and the mean taken off the ratio
-  // (device; nullptr: 0)
-  const float* h0 = nullptr;
-  const float* mean = nullptr;
+  // paired passes: what the second convolution made of the mean taken off the
+  // ratio (device)
+  const float* add = nullptr;
 };
 
 // ---------------------------------------------------------------- passes
@@ -147,7 +146,7 @@ int launch_z_pass(const Geom& g, const FftLen& fz, float2* S, const OtfDev& otf,
                   cudaStream_t st, bool fwd_only = false);
 // Inverse x pass followed by the RL ratio and the forward x pass of the
 // second convolution (spectrum updated in place).
-// The paired pass takes *mean (nullptr: 0) off the ratio before the transform.
+// The paired pass takes *mean off the ratio before the transform.
 int launch_x_inv_ratio_fwd(const Geom& g, const FftLen& fx, float2* S, const float* raw,
                            const float* mean, float eps, cudaStream_t st);
 // Inverse x pass followed by the estimate update from the prediction Y:
