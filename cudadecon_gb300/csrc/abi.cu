@@ -435,7 +435,7 @@ static int rl_loop(const GridPlan& p, const LoopBufs& b, int nIter, cudaStream_t
     mark();
     if ((rc = launch_x_fwd(g, p.fx, X, Xm1, lam_k, predict, b.S, st))) return rc;
     mark();
-    if ((rc = launch_y_pass(g, p.fy, b.S, false, st))) return rc;
+    if ((rc = launch_y_pass(g, p.fy, b.S, false, st, true))) return rc;
     mark();
     if ((rc = launch_z_pass(g, p.fz, b.S, p.otf, false, st))) return rc;
     mark();
@@ -1650,7 +1650,7 @@ int cdx_rfft3d_device(const float* in, void* out_complex, int nx, int ny, int nz
              fft_len_init(fz, nz, Axis::z) || S.ensure((size_t)g.spec_elems()));
   if (ok) choose_layout(g, fx, fy);
   ok = ok && !(launch_x_fwd(g, fx, in, nullptr, nullptr, 0, S.p, st) ||
-             launch_y_pass(g, fy, S.p, false, st) || launch_z_pass(g, fz, S.p, none, false, st, true) ||
+             launch_y_pass(g, fy, S.p, false, st, true) || launch_z_pass(g, fz, S.p, none, false, st, true) ||
              launch_spec_to_std(g, S.p, (float2*)out_complex, st) || cudaStreamSynchronize(st));
   fft_len_free(fx);
   fft_len_free(fy);
@@ -1672,7 +1672,7 @@ int cdx_conv3d_device(const float* in, float* out, int nx, int ny, int nz, int c
   DevBuf<float2> S;
   int ok = !(S.ensure((size_t)p.g.spec_elems()) ||
              launch_x_fwd(p.g, p.fx, in, nullptr, nullptr, 0, S.p, st) ||
-             launch_y_pass(p.g, p.fy, S.p, false, st) ||
+             launch_y_pass(p.g, p.fy, S.p, false, st, true) ||
              launch_z_pass(p.g, p.fz, S.p, p.otf, conj != 0, st) ||
              launch_y_pass(p.g, p.fy, S.p, true, st) || launch_x_inv_plain(p.g, p.fx, S.p, out, st) ||
              cudaStreamSynchronize(st));
@@ -1792,7 +1792,7 @@ int cdx_wiener_device(const float* in, float* out, int nx, int ny, int nz, float
            launch_wiener_h(g, s.raw_otf.p, (int)s.od.nx_otf, (int)s.od.nz_otf, dkx, dky, kxscale,
                            kyscale, kzscale, rcutoff, w, H, st) ||
            launch_x_fwd(g, p.fx, x, nullptr, nullptr, 0, S, st, g.pair ? background : 0.f) ||
-           launch_y_pass(g, p.fy, S, false, st) || launch_z_pass(g, p.fz, S, hd, false, st) ||
+           launch_y_pass(g, p.fy, S, false, st, true) || launch_z_pass(g, p.fz, S, hd, false, st) ||
            launch_y_pass(g, p.fy, S, true, st) || launch_x_inv_plain(g, p.fx, S, out, st));
     // also after a failure: earlier passes may still be using the workspaces
     ok = cudaStreamSynchronize(st) == cudaSuccess && ok;

@@ -349,7 +349,7 @@ k_px_ratio(PairGeom g, const float2* __restrict__ tw, float4* S, const float* __
   extern __shared__ __align__(16) float2 smem[];
   float2* stw = smem;
   float4* sm = P::tile(smem);
-  const int z = blockIdx.y, m0 = blockIdx.x * NQ;
+  const int z = slice_of_block(g), m0 = blockIdx.x * NQ;
   copy_twiddles<P::kTw>(tw, stw);
   prefetch_rows<NQ>(g, P::rows(smem, 0), raw, z, m0);  // written before the iterations
   cp_async_commit();
@@ -434,7 +434,7 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
   __shared__ float4 red[32];
   float2* stw = smem;
   float4* sm = P::tile(smem);
-  const int z = blockIdx.y, m0 = blockIdx.x * NQ;
+  const int z = slice_of_block(g), m0 = blockIdx.x * NQ;
   copy_twiddles<P::kTw>(tw, stw);
   cp_async_commit();
   const RowRuns<NQ> runs(g, z, m0);

@@ -51,7 +51,9 @@ int launch_x_inv_update(const Geom& g, const FftLen& fx, const float2* S, const 
                         cudaStream_t st) {
   if (g.pair) {
     bool done = false;
-    const int rc = pxgen_update(pair_geom(g), fx.d_pair, S, Y, Xout, G, dots, &w, lam_next, eps, st,
+    PairGeom pg = pair_geom(g);
+    pg.down = past_l2(g);
+    const int rc = pxgen_update(pg, fx.d_pair, S, Y, Xout, G, dots, &w, lam_next, eps, st,
                                 &done);
     if (done || rc) return rc;
   }

@@ -52,8 +52,13 @@ static int y_dispatch(const Geom& g, const FftLen& fy, float2* S, cudaStream_t s
   return y_go<INV, GenericRunner>(g, fy.dev, S, V, threads_for((long long)V * g.ny), st);
 }
 
-int launch_y_pass(const Geom& g, const FftLen& fy, float2* S, bool inverse, cudaStream_t st) {
-  if (g.pair) return launch_py(pair_geom(g), fy, S, inverse, st);
+int launch_y_pass(const Geom& g, const FftLen& fy, float2* S, bool inverse, cudaStream_t st,
+                  bool after_fwd) {
+  if (g.pair) {
+    PairGeom pg = pair_geom(g);
+    pg.down = after_fwd && past_l2(g);
+    return launch_py(pg, fy, S, inverse, st);
+  }
   return inverse ? y_dispatch<true>(g, fy, S, st) : y_dispatch<false>(g, fy, S, st);
 }
 

@@ -138,8 +138,10 @@ int x_pass_blocks(const Geom& g);
 // subtracted from X (paired layout without prediction only).
 int launch_x_fwd(const Geom& g, const FftLen& fx, const float* X, float* Xm1,
                  const float* lam, int predict, float2* S, cudaStream_t st, float bg = 0.f);
-// In-place complex FFT along y of every (kx, z) row.
-int launch_y_pass(const Geom& g, const FftLen& fy, float2* S, bool inverse, cudaStream_t st);
+// In-place complex FFT along y of every (kx, z) row.  after_fwd: launch_x_fwd wrote
+// the spectrum (the order in which the slices are taken follows it).
+int launch_y_pass(const Geom& g, const FftLen& fy, float2* S, bool inverse, cudaStream_t st,
+                  bool after_fwd = false);
 // z FFT, multiply by OTF (or its conjugate), inverse z FFT, in place.
 // fwd_only (test path) stops after the forward z FFT.
 int launch_z_pass(const Geom& g, const FftLen& fz, float2* S, const OtfDev& otf, bool conj,

@@ -288,7 +288,7 @@ static int make_otf_device(float* d_psf, int nx, int ny, int nz, const OtfMakePa
   OTF_CHECK(cudaMalloc(&d_S, sizeof(float2) * (size_t)g.spec_elems()));
   OTF_CHECK(cudaMalloc(&d_std, sizeof(float2) * (size_t)nxh * ny * nz));
   if (launch_x_fwd(g, fx, d_psf, nullptr, nullptr, 0, d_S, st) ||
-      launch_y_pass(g, fy, d_S, false, st) || launch_z_pass(g, fz, d_S, none, false, st, true) ||
+      launch_y_pass(g, fy, d_S, false, st, true) || launch_z_pass(g, fz, d_S, none, false, st, true) ||
       launch_spec_to_std(g, d_S, d_std, st)) {
     cleanup_all();
     return cudaErrorLaunchFailure;
