@@ -132,7 +132,10 @@ static std::vector<int> pair_radices(int L, Axis axis, int& points) {
 // exp(-2 pi i k / L) of the step across the lanes follow, k < L / 2.
 static int build_pair(FftLen& f, int L, int points, const std::vector<int>& rad) {
   FftDev d;
-  if (points == L) return build_fft_dev(L, rad, d, &f.d_pair);
+  if (points == L) {
+    f.pair_kc = L / rad.back();
+    return build_fft_dev(L, rad, d, &f.d_pair);
+  }
   float2* plan = nullptr;
   if (int rc = build_fft_dev(points, rad, d, &plan)) return rc;
   std::vector<float2> w(points);
@@ -191,6 +194,7 @@ void choose_layout(Geom& g, const FftLen& fx, const FftLen& fy) {
   const bool s_fits = (long long)pair_half(g.ny) * 2 * g.nxh < (1LL << 31);
   g.pair = fx.d_pair && z_fits && s_fits && pair_rows(g.ny) && !(dft_form() == 1 && fx.has_tc);
   g.eo = g.pair && fy.d_pair && fy.pair_eo;
+  g.kc = g.pair && fy.d_pair && !fy.pair_eo ? fy.pair_kc : 0;
 }
 
 int tc_check(const FftLen& f) {
@@ -215,7 +219,7 @@ void fft_len_free(FftLen& f) {
   }
   f.dev.tw = f.sdev.tw = f.gzdev.tw = nullptr;
   f.has_static = f.has_gz = false;
-  f.pair_eo = 0;
+  f.pair_eo = f.pair_kc = 0;
   if (f.has_tc) tc_tables_free(f.tc);
   f.has_tc = false;
 }

@@ -90,7 +90,11 @@ k_py_gen(PairGeom g, FftDev fy, float4* S4, int V) {
 
 template <bool INV>
 static int py_gen_go(const PairGeom& g, const FftLen& fy, float2* S, cudaStream_t st) {
+  // rows per block: about 2048 elements, fewer where that leaves the chip idle
+  // (64 x 2 x 256: 14 us a pass with 1024 rows in each of 9 blocks)
+  const long long rows_per_block = (long long)g.nxh * g.nz / (4 * sm_count());
   int V = 2048 / g.ny;
+  if (V > rows_per_block) V = (int)rows_per_block;
   if (V < 1) V = 1;
   const size_t smem = sizeof(float2) * ((size_t)g.ny + spad_size(V * g.ny));
   const long long nrows = (long long)g.nxh * g.nz;

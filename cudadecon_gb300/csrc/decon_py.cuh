@@ -102,8 +102,36 @@ k_py_eo(PairGeom g, const float2* __restrict__ tw, float4* S) {
   const bool self = self_row(g, kxa);
   grid_dep_wait();
   if (!INV) {
+    if constexpr (!kSame) {
+      // rows m and m + HP belong to different butterflies: they go through the
+      // tile, so that every slot is read once (each butterfly reading its half of
+      // the slots it needs took 86 us on 96 x 486 x 525, all from DRAM twice)
+      constexpr int kSlots = round_up(HP, 4) * V, N = (kSlots + P::T - 1) / P::T;
+      C2 zp[N], zm[N];
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        int m, v;
+        slot_order<V, 4>(idx + n * P::T, m, v);
+        if (m >= HP || kx0 + v >= g.nxh) continue;
+        zp[n] = ldp(slot(kx0 + v, m, StepA{}, 0));
+        zm[n] = self_row(g, kx0 + v) ? zp[n] : ldp(slot(kx0 + v, g.hp + m, StepA{}, 0));
+      }
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        int m, v;
+        slot_order<V, 4>(idx + n * P::T, m, v);
+        if (m >= HP || kx0 + v >= g.nxh) continue;
+        C2 a, b;
+        split_rows(zp[n], zm[n], a, b);
+        float4* t = sm + v * PL::VS;
+        stp(t + PL::pos(m), a);
+        if (m + HP < PL::L) stp(t + PL::pos(m + HP), b);
+      }
+      __syncthreads();
+    }
     if (act_a) {
       C2 x[Q0];
+      float4* p = sm + va * PL::VS + j;
       if constexpr (kSame) {
 #pragma unroll
         for (int r = 0; r < Q0 / 2; ++r) {
@@ -112,21 +140,10 @@ k_py_eo(PairGeom g, const float2* __restrict__ tw, float4* S) {
           split_rows(zp, zm, x[r], x[r + Q0 / 2]);
         }
       } else {
-        // each butterfly takes its half of every slot it needs
 #pragma unroll
-        for (int r = 0; r < Q0; ++r) {
-          const int e = j + r * PL::KA;
-          const bool second = e >= HP;
-          const int m = second ? e - HP : e;
-          const C2 zp = ldp(slot(kxa, m, StepA{}, 0));
-          const C2 zm = self ? zp : ldp(slot(kxa, g.hp + m, StepA{}, 0));
-          C2 a, b;
-          split_rows(zp, zm, a, b);
-          x[r] = second ? b : a;
-        }
+        for (int r = 0; r < Q0; ++r) x[r] = ldp(p + r * PL::S0);
       }
       PDft<Q0, false>::run(x);
-      float4* p = sm + va * PL::VS + j;
 #pragma unroll
       for (int r = 0; r < Q0; ++r) stp(p + r * PL::S0, x[r]);
     }
@@ -240,23 +257,29 @@ __device__ __forceinline__ void swap_lanes(C2& a, C2& b) {
 
 template <class PL, int V>
 struct PYZ {
-  static constexpr int T = PL::threads(V);
+  static constexpr int KC4 = round_up(PL::KC, 4);
+  static constexpr int kmax = PL::kmax() > KC4 ? PL::kmax() : KC4;
+  static constexpr int T = round_up(V * kmax, 32);
   static constexpr int kTw = PL::L + (PL::L & 1);
   static constexpr size_t kSmem = sizeof(float2) * kTw + sizeof(float4) * V * PL::VS;
 };
 
-// Global memory is read and written a slot (two rows or two columns) at a
-// time, and the tile regroups the lanes: a round trip each on the way in and
-// out.  Only the inverse's columns are read by the butterflies themselves, each
-// picking its lane of the slot (two threads share one, so a warp's loads stay
-// coalesced): 22.5 us on 126 x 189 x 324 against 25.0 regrouped; for the rows of
-// the forward pass, which come as two slots each, that took 32.6 against 23.5.
+// The rows are read and written a slot (two of them) at a time, and the tile
+// regroups the lanes: a round trip more than an even height on the way in of the
+// forward and out of the inverse transform.  Its columns go straight between
+// registers and memory: a slot pairs the columns k and k + KC of one stage C
+// butterfly (pair_layout.cuh), and the odd one left over of each butterfly goes
+// with its neighbour's, by a shuffle.  With slots of neighbouring columns
+// (2p, 2p + 1) the forward pass regrouped once more and the inverse read every
+// slot twice.
 template <class PL, int V, bool INV>
-__global__ void __launch_bounds__(PYZ<PL, V>::T, PL::blocks_of(PYZ<PL, V>::T, 40))
+__global__ void __launch_bounds__(PYZ<PL, V>::T, PL::blocks_of(PYZ<PL, V>::T, 28))
 k_py_zz(PairGeom g, const float2* __restrict__ tw, float4* S) {
   using P = PYZ<PL, V>;
-  constexpr int Q0 = PL::Q0, Q2 = PL::Q2, L = PL::L, H = pair_split(L), T = P::T;
-  constexpr int kRows = H / 2, kCols = (L + 1) / 2;  // slots of a half row, of a row of columns
+  constexpr int Q0 = PL::Q0, Q2 = PL::Q2, L = PL::L, H = pair_split(L), T = P::T, KC = PL::KC;
+  constexpr int kRows = H / 2;            // slots of a half row
+  constexpr int KS = pair_kcs(L, KC), kFull = (Q2 - 1) / 2 * KS;  // slots of two columns of one butterfly
+  static_assert(Q2 % 2 == 1, "an odd length");
   extern __shared__ __align__(16) float2 smem[];
   float2* stw = smem;
   float4* sm = reinterpret_cast<float4*>(smem + P::kTw);
@@ -270,31 +293,40 @@ k_py_zz(PairGeom g, const float2* __restrict__ tw, float4* S) {
   const long long dz = two ? g.zstep : 0;
   const int half = g.hp * g.nxh;  // slots to the mirrored half
   auto at = [&](int v, int s) { return slice + ((s >> 2) * g.nxh + kx0 + v) * 4 + (s & 3); };
-  // lane e & 1 of both slices' slots at p
-  auto pick = [&](const float4* p, int e) {
-    const float4 u = *p, w = p[dz];
-    return e & 1 ? C2{make_float2(u.y, w.y), make_float2(u.w, w.w)}
-                 : C2{make_float2(u.x, w.x), make_float2(u.z, w.z)};
-  };
   const int va = idx / PL::KA, j = idx - va * PL::KA;
-  const int vc = idx / PL::KC, k = idx - vc * PL::KC;
   float4* pa = sm + va * PL::VS + j;
-  float4* pc = sm + vc * PL::VS + pos_c<PL>(k);
-  auto pos_f = [](int f) {  // frequency f of a vector, as stage C holds it
-    const int r = f / PL::KC;
-    return pos_c<PL>(f - r * PL::KC) + r;
-  };
+  // stage C: 4 neighbouring k, then the next kx, then the next 4 k
+  int k, vc;
+  slot_order<V, 4>(idx, k, vc);
+  const bool act_c = k < KC && kx0 + vc < g.nxh;
+  // the left over column and its partner's (k = KC, past the end, has none of its own)
+  const bool act_l = k <= KC && kx0 + vc < g.nxh, odd = k & 1;
+  float4* pc = sm + vc * PL::VS + (k < KC ? pos_c<PL>(k) : 0);
+  auto swap = [](float v) { return __shfl_xor_sync(0xffffffffu, v, 1); };
   if (!INV) {
-    for (int i = idx; i < (kRows + 3) / 4 * 4 * V; i += T) {
+    // all loads of a thread's slots before the first is used
+    constexpr int kSlots = round_up(kRows, 4) * V, N = (kSlots + T - 1) / T;
+    C2 p0[N], p1[N], m0[N], m1[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
       int m, v;
-      slot_order<V, 4>(i, m, v);
+      slot_order<V, 4>(idx + n * T, m, v);
       if (m >= kRows || kx0 + v >= g.nxh) continue;
       const bool self = self_row(g, kx0 + v);
       const float4* src = at(v, m);
-      const C2 p0 = ldp(src), p1 = ldp(src + dz);
+      p0[n] = ldp(src);
+      p1[n] = ldp(src + dz);
+      m0[n] = self ? p0[n] : ldp(src + half);
+      m1[n] = self ? p1[n] : ldp(src + half + dz);
+    }
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      int m, v;
+      slot_order<V, 4>(idx + n * T, m, v);
+      if (m >= kRows || kx0 + v >= g.nxh) continue;
       C2 a0, b0, a1, b1;
-      split_rows(p0, self ? p0 : ldp(src + half), a0, b0);
-      split_rows(p1, self ? p1 : ldp(src + half + dz), a1, b1);
+      split_rows(p0[n], m0[n], a0, b0);
+      split_rows(p1[n], m1[n], a1, b1);
       swap_lanes(a0, a1);
       swap_lanes(b0, b1);
       float4* t = sm + v * PL::VS;
@@ -317,38 +349,50 @@ k_py_zz(PairGeom g, const float2* __restrict__ tw, float4* S) {
     __syncthreads();
     stage_b<PL, V, false, false>(sm, stw);
     grid_dep_launch_small();
-    if (vc < V) {
-      C2 x[Q2];
+    C2 x[Q2];
+    if (act_c) {
 #pragma unroll
       for (int r = 0; r < Q2; ++r) x[r] = ldp(pc + r);
-      butterfly<Q2, PL::KC, false, false>(x, stw, k);
+      butterfly<Q2, KC, false, false>(x, stw, k);
 #pragma unroll
-      for (int r = 0; r < Q2; ++r) stp(pc + r, x[r]);
+      for (int r = 0; r + 1 < Q2; r += 2) {
+        swap_lanes(x[r], x[r + 1]);
+        float4* dst = at(vc, r / 2 * KS + k);
+        stp(dst, x[r]);
+        if (two) stp(dst + dz, x[r + 1]);
+      }
+    } else {
+      x[Q2 - 1] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
     }
-    __syncthreads();
-    for (int i = idx; i < (kCols + 3) / 4 * 4 * V; i += T) {
-      int s, v;
-      slot_order<V, 4>(i, s, v);
-      if (s >= kCols || kx0 + v >= g.nxh) continue;
-      const float4* t = sm + v * PL::VS;
-      C2 a = ldp(t + pos_f(2 * s)), b = 2 * s + 1 < L ? ldp(t + pos_f(2 * s + 1)) : a;
-      swap_lanes(a, b);
-      stp(at(v, s), a);
-      if (two) stp(at(v, s) + dz, b);
+    // even k: slice 0 of columns k and k + 1; odd k: slice 1 of k - 1 and k
+    const C2 u = x[Q2 - 1];
+    const float re = swap(odd ? u.re.x : u.re.y), im = swap(odd ? u.im.x : u.im.y);
+    if (act_l && (two || !odd)) {
+      float4* dst = at(vc, kFull + (k >> 1));
+      stp(odd ? dst + dz : dst, odd ? C2{make_float2(re, u.re.y), make_float2(im, u.im.y)}
+                                    : C2{make_float2(u.re.x, re), make_float2(u.im.x, im)});
     }
   } else {
     C2 x[Q2];
-    if (vc < V && kx0 + vc < g.nxh) {
+    if (act_c) {
 #pragma unroll
-      for (int r = 0; r < Q2; ++r) {
-        const int f = k + r * PL::KC;
-        x[r] = pick(at(vc, f >> 1), f);
+      for (int r = 0; r + 1 < Q2; r += 2) {
+        const float4* src = at(vc, r / 2 * KS + k);
+        x[r] = ldp(src);
+        x[r + 1] = ldp(src + dz);
       }
     }
+    C2 u = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    if (act_l) u = ldp(at(vc, kFull + (k >> 1)) + (odd ? dz : 0));
+    const float re = swap(odd ? u.re.x : u.re.y), im = swap(odd ? u.im.x : u.im.y);
+    x[Q2 - 1] = odd ? C2{make_float2(re, u.re.y), make_float2(im, u.im.y)}
+                    : C2{make_float2(u.re.x, re), make_float2(u.im.x, im)};
     cp_async_wait_all();
     __syncthreads();
-    if (vc < V) {
-      butterfly<Q2, PL::KC, true, true>(x, stw, k);
+    if (act_c) {
+#pragma unroll
+      for (int r = 0; r + 1 < Q2; r += 2) swap_lanes(x[r], x[r + 1]);
+      butterfly<Q2, KC, true, true>(x, stw, k);
 #pragma unroll
       for (int r = 0; r < Q2; ++r) stp(pc + r, x[r]);
     }

@@ -30,8 +30,8 @@ struct Geom {
   int nyp;         // ny rounded up to even
   long long plane; // nz * nyp complex elements per kx plane
   // 1: the spectrum is in the paired layout (pair_layout.cuh) and the paired
-  // passes run; eo: that layout's column order (choose_layout)
-  int pair = 0, eo = 0;
+  // passes run; eo, kc: that layout's column order (choose_layout)
+  int pair = 0, eo = 0, kc = 0;
   long long nvox() const { return (long long)nx * ny * nz; }
   // complex elements of a buffer that holds either layout
   long long spec_elems() const {
@@ -101,9 +101,9 @@ struct FftLen {
   FftDev gzdev;
   float2* d_twgz = nullptr;
   // twiddles of the paired plan (fft_pair.cuh), if the length has one; y: the
-  // column order it leaves (PairGeom::eo)
+  // column order it leaves (PairGeom::eo, kc)
   float2* d_pair = nullptr;
-  int pair_eo = 0;
+  int pair_eo = 0, pair_kc = 0;
   // the tensor-core plan of the length, if it has one
   bool has_tc = false;
   TcTables tc;

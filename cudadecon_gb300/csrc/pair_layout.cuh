@@ -12,7 +12,10 @@
 //                               slot hp + m      Z[-kx] of pair m,
 //   after the forward y pass:   the columns ky of the half spectrum, two per
 //                               slot: (k, k + ny/2) where the y pass splits
-//                               even and odd rows (eo), else (2p, 2p + 1).
+//                               even and odd rows (eo); (k + 2q kc, k + (2q + 1)
+//                               kc) of one butterfly of an odd height's plan, its
+//                               last kc columns as neighbours (kc); else (2p,
+//                               2p + 1).
 // A slot holds (re lane 0, re lane 1, im lane 0, im lane 1).  Row 0 and, for
 // even nx, row nx/2 are their own mirror image and leave the second half
 // unused.
@@ -34,10 +37,22 @@ struct PairGeom {
   int H, hp;   // row y shares a complex row with y + H; slots per half row
   int sb;      // blocks of 4 slots per row: hp / 2
   int slots;   // column pairs after the y pass
-  int eo;      // 1: columns (k, k + ny/2), 0: (2p, 2p + 1)
+  int eo;      // 1: columns (k, k + ny/2)
+  int kc;      // > 0: columns (k + 2q kc, k + (2q + 1) kc); neither: (2p, 2p + 1)
+  int kcs, full;  // slots from one q to the next, slots of such pairs
+  int last;       // first of the last kc columns, less 2 full
+  float inv_kcs;
   int zstep;   // slots per z: sb * nxh * 4
   int down = 0;  // 1: the pass takes the slices from the last to the first
-  __host__ __device__ int col(int s, int lane) const { return eo ? s + lane * (ny >> 1) : 2 * s + lane; }
+  // columns of slot s; ny and more: none.  (The quotient is exact: s + 1/2 lies
+  // farther from the multiples of kcs than s < 2^20 rounds.)
+  __host__ __device__ int col_step(int s) const { return eo ? ny >> 1 : s >= full ? 1 : kc; }
+  __host__ __device__ int col(int s, int lane) const {
+    if (eo) return s + lane * (ny >> 1);
+    if (s >= full) return 2 * s + lane + last;
+    const int q = (int)(((float)s + 0.5f) * inv_kcs), k = s - q * kcs;
+    return k < kc ? k + (2 * q + lane) * kc : ny;
+  }
   // slot s of row (kx, z)
   __host__ __device__ long long slot(int kx, int z, int s) const {
     return (long long)z * zstep + ((long long)(s >> 2) * nxh + kx) * 4 + (s & 3);
@@ -46,12 +61,30 @@ struct PairGeom {
   // part is two floats further
   __host__ __device__ long long at(int kx, int z, int ky) const {
     const int h = ny >> 1;
-    const int s = eo ? (ky < h ? ky : ky - h) : ky >> 1;
-    const int lane = eo ? ky >= h : ky & 1;
+    int s = ky >> 1, lane = ky & 1;
+    if (eo) {
+      lane = ky >= h;
+      s = ky - lane * h;
+    } else if (kc) {
+      const int r = ky / kc, k = ky - r * kc;
+      if (r == ny / kc - 1) {
+        lane = k & 1;
+        s = full + (k >> 1);
+      } else {
+        lane = r & 1;
+        s = (r >> 1) * kcs + k;
+      }
+    }
     return 4 * slot(kx, z, s) + lane;
   }
 };
 
+// Slots from the first column of a stage C output pair to the next pair's: kc, or
+// whole blocks of 4 where the row has room for the slots that leaves empty.
+__host__ __device__ inline constexpr int pair_kcs(int ny, int kc) {
+  const int up = (kc + 3) / 4 * 4;
+  return kc && (ny / kc - 1) / 2 * up + (kc + 1) / 2 <= 2 * pair_half(ny) ? up : kc;
+}
 // Whether the arrays of an iteration are past what L2 holds of them.  Each pass
 // then takes the slices in the order opposite to the one that wrote them, so that
 // it finds the last ones still there: x forward up, y forward down, z, y inverse
@@ -71,6 +104,12 @@ inline PairGeom pair_geom(const Geom& g) {
   p.sb = p.hp / 2;
   p.slots = (g.ny + 1) / 2;
   p.eo = g.eo;
+  p.kc = g.kc;
+  p.kcs = pair_kcs(g.ny, g.kc);
+  p.full = g.kc ? (g.ny / g.kc - 1) / 2 * p.kcs : 0;
+  p.last = g.kc ? g.ny - g.kc - 2 * p.full : 0;
+  p.inv_kcs = g.kc ? 1.f / (float)p.kcs : 0.f;
+  if (g.kc) p.slots = p.full + (g.kc + 1) / 2;
   p.zstep = p.sb * g.nxh * 4;
   return p;
 }

@@ -4,7 +4,7 @@ csrc/static_plans.cuh does not already hold: x in [128, 1024], y in
 [128, 512], z in [32, 160].
 
 Writes csrc/static_plans_gen.cuh (those plan lists), and for the paired passes
-of the plain form (csrc/fft_pair.cuh; x in [128, 2048], y in [32, 1024], z in
+of the plain form (csrc/fft_pair.cuh; x in [128, 2048], y in [8, 2048], z in
 [16, 256]) csrc/pair_plans_gen.cuh (the plans), csrc/x_gen_dispatch.h (their
 dispatch) and csrc/decon_{x,y,z}_gen_<k>.cu (their kernels, spread over several
 units so that the build compiles them in parallel).
@@ -319,13 +319,22 @@ def choose(axis: str, L: int, column: int | None,
 
 # ---------------------------------------------------------------- paired plans
 PAIR_X_RANGE = (128, 2048)
-PAIR_Y_RANGE = (32, 1024)
+PAIR_Y_RANGE = (8, 2048)
 PAIR_Z_RANGE = (16, 256)
 PAIR_MAX_RADIX = 16
 PAIR_Y_RADIX = 18  # y 324 as 18 9 took 30-37 us a pass on 108 x 324 x 525, as 6 9 3 35-44 us
 PAIR_X_RADIX = 12  # x 256 as 4 8 8 took 17 us in x ratio, as 16 16 30 us
-PAIR_WIDE_RADIX = 27
+PAIR_THREE_RADIX = 27
+# odd heights: two radices to 35 where three need one above 9 (each round trip costs
+# an odd height more: 525 as 25 21 took 30 us a pass on 64 x 525 x 384, as 7 15 5 45)
+PAIR_WIDE_RADIX = 35
 PAIRP = HERE / "csrc" / "pair_plans_gen.cuh"
+
+
+def pair_two(L: int, most: int) -> tuple[int, int, int] | None:
+    """The most balanced two radices of at most `most` points, larger first."""
+    c = [(a, 1, L // a) for a in range(2, most + 1) if L % a == 0 and 2 <= L // a <= a]
+    return min(c, default=None)
 
 
 def pair_lengths() -> dict[str, list[int]]:
@@ -348,14 +357,14 @@ def pair_radices(L: int, even_first: bool, most: int = PAIR_MAX_RADIX) -> tuple[
     is even.  Radices up to `most` or 16 and then 27 where that leaves no plan (625 = 5 25 5); None
     where that does not either (1715 = 5 7^3)."""
     best = None
-    for a in range(2, PAIR_WIDE_RADIX + 1):
+    for a in range(2, PAIR_THREE_RADIX + 1):
         if L % a:
             continue
-        for b in range(1, PAIR_WIDE_RADIX + 1):
+        for b in range(1, PAIR_THREE_RADIX + 1):
             if (L // a) % b:
                 continue
             c = L // a // b
-            if not 2 <= c <= PAIR_WIDE_RADIX or (even_first and a % 2):
+            if not 2 <= c <= PAIR_THREE_RADIX or (even_first and a % 2):
                 continue
             two, m = b == 1, max(a, b, c)
             key = (m > most, m > max(most, PAIR_MAX_RADIX), not two, m, 0 if two else -min(a, b, c), c, -b)
@@ -374,25 +383,34 @@ def _slots(addr: np.ndarray) -> int:
 
 
 @functools.lru_cache(maxsize=None)
-def pair_strides(L: int, rad: tuple[int, int, int], V: int, axis: str, run: int) -> tuple[int, int]:
+def pair_strides(L: int, rad: tuple[int, int, int], V: int, axis: str, odd: bool) -> tuple[int, int]:
     """Strides (S0 of the first digit, VS of a vector) of the shared tile with
     the fewest modelled wavefronts over the three stages' accesses, smallest
     first.  x: stage A's threads run over the vectors first.  y: the threads
-    of stages A and C run over `run` butterflies, then the vectors; run = 1
-    (odd heights): vectors slowest, and S0 = Q1 Q2, so that the regrouping
-    passes address elements without a division."""
+    of stages A and C run over 4 butterflies, then the vectors; odd heights:
+    those of stage A over a vector, those that regroup rows over 4 pairs of
+    rows, then the vectors."""
     q0, q1, q2 = rad
     ka, kb, kc = q1 * q2, q0 * q2, q0 * q1
     best = None
-    for s0 in range(ka, ka + (1 if run == 1 else 8)):
+    def runs(n):  # 4 consecutive, then the vectors
+        i = np.arange(V * (n // 4) * 4)
+        return i // (4 * V) * 4 + i % 4, i // 4 % V
+
+    for s0 in range(ka, ka + 8):
         for vs in range((q0 - 1) * s0 + ka, (q0 - 1) * s0 + ka + (8 if V > 1 else 1)):
+            i = np.arange(V * ka)
             if axis == "x":
-                i = np.arange(V * ka)
                 j, v = i // V, i % V
+            elif odd:
+                j, v = i % ka, i // ka
             else:
-                i = np.arange(V * (ka // run) * run)
-                j, v = (i // (run * V) * run + i % run, i // run % V) if run > 1 else (i % ka, i // ka)
+                j, v = runs(ka)
             cost = q0 * _slots(v * vs + j)
+            if odd:
+                m, v = runs(L // 4)
+                for e in (2 * m, 2 * m + 1):
+                    cost += 2 * _slots(v * vs + e // ka * s0 + e % ka)
             if q1 > 1:
                 i = np.arange(V * kb)
                 v, w = i // kb, i % kb
@@ -401,8 +419,7 @@ def pair_strides(L: int, rad: tuple[int, int, int], V: int, axis: str, run: int)
                 i = np.arange(V * kc)
                 v, k = i // kc, i % kc
             else:
-                i = np.arange(V * (kc // run) * run)
-                k, v = (i // (run * V) * run + i % run, i // run % V) if run > 1 else (i % kc, i // kc)
+                k, v = runs(kc)
             cost += q2 * _slots(v * vs + k % q0 * s0 + k // q0 * q2)
             key = (cost, vs)
             if best is None or key < best[0]:
@@ -434,21 +451,44 @@ def pair_z_warps(L: int, rad, V: int) -> int:
     return min(65536 // (t * (4 * max(rad) + 56)), 227 * 1024 // (8 * L + 32 * V * L + 1024)) * t // 32
 
 
+def pair_y_odd_kx(L: int, two: bool) -> int:
+    """Neighbouring kx per block of an odd height: few, since every round trip
+    ends at a barrier (64 x 441 x 384: 23 us a pass with 2, 25 with 4, 31 with 8),
+    but more where two radices leave few threads per kx (225: 16 us with 4, 19
+    with 2) and one where three radices make a block of many (1215: 35 with 1, 41
+    with 2 on 32 x 1215 x 384)."""
+    if L < 100:
+        return 8
+    if L <= (384 if two else 180):
+        return 4
+    return 2 if two or L < 1000 else 1
+
+
 def pair_plan(axis: str, L: int) -> tuple[int, int, tuple[int, int, int], int, int]:
     """(transform length, vectors per block, radices, S0, VS) of one length.
     x: 2 pairs (half a slot block of the layout), 4 where that
     keeps more warps on an SM (810 at 180 slices of 600 rows: x ratio 308 us
-    with 4, 390 with 2; 1024: 282 and 234); y: neighbouring kx for about 128 threads; z: 16 column pairs
+    with 4, 390 with 2; 1024: 282 and 234); y: neighbouring kx for about 128 threads
+    at even heights; z: 16 column pairs
     (256-byte runs), 8 where that keeps more warps on an SM."""
     if axis == "x":
         rad = pair_radices(L, False, PAIR_X_RADIX)
         V = 4 if pair_x_warps(L, rad, 4) > 1.1 * pair_x_warps(L, rad, 2) else 2
-        return (L, V, rad, *pair_strides(L, rad, V, "x", 0))
+        return (L, V, rad, *pair_strides(L, rad, V, "x", False))
     if axis == "y":
         n, even = pair_y_points(L)
         rad = pair_radices(n, even, PAIR_Y_RADIX)
-        V = max(4, round(128 / pair_threads(rad, 8) * 8))
-        return (n, V, rad, *pair_strides(n, rad, V, "y", 4 if n != L else 1))
+        if n == L:
+            if max(rad) > 9 and rad[1] > 1:
+                rad = pair_two(n, PAIR_WIDE_RADIX) or rad
+            V = pair_y_odd_kx(n, rad[1] == 1)
+        else:
+            # two where four take more than 256 threads (810: 50 and 38 us a pass
+            # against 51 and 45 on 64 x 810 x 384; 1024, 256 threads: 47 us with 4, 49 with 2)
+            V = max(4, round(128 / pair_threads(rad, 8) * 8)) & ~1
+            if pair_threads(rad, V) > 256:
+                V = 2
+        return (n, V, rad, *pair_strides(n, rad, V, "y", n == L))
     rad = pair_radices(L, False)
     V = 8 if pair_z_warps(L, rad, 8) > 1.2 * pair_z_warps(L, rad, 16) else 16
     return (L, V, rad, rad[1] * rad[2], L)
