@@ -1,5 +1,5 @@
 // Generated by cudadecon_gb300/gen_plans.py (do not edit): paired z-pass kernels
-// of the lengths 16, 30, 49, 72, 100, 135, 175, 224.
+// of the lengths 16, 30, 49, 72, 100, 135, 175, 224, 270, 336, 400, 486.
 #include "decon_pz.cuh"
 #include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
@@ -28,10 +28,22 @@ int pzgen_0(const PairGeom& g, const float2* tw, float2* S, const OtfDev& otf, b
       return pz_mode<PPZ135, 16>(g, tw, S, otf, conj, st, fwd_only);
     case 175:
       *done = true;
-      return pz_mode<PPZ175, 16>(g, tw, S, otf, conj, st, fwd_only);
+      return pz_mode<PPZ175, 8>(g, tw, S, otf, conj, st, fwd_only);
     case 224:
       *done = true;
       return pz_mode<PPZ224, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 270:
+      *done = true;
+      return pz_mode<PPZ270, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 336:
+      *done = true;
+      return pz_mode<PPZ336, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 400:
+      *done = true;
+      return pz_mode<PPZ400, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 486:
+      *done = true;
+      return pz_mode<PPZ486, 8>(g, tw, S, otf, conj, st, fwd_only);
     default:
       return 0;
   }

@@ -1,5 +1,5 @@
 // Generated by cudadecon_gb300/gen_plans.py (do not edit): paired z-pass kernels
-// of the lengths 21, 36, 56, 81, 112, 147, 192, 243.
+// of the lengths 21, 36, 56, 81, 112, 147, 192, 243, 294, 360, 432, 504.
 #include "decon_pz.cuh"
 #include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
@@ -28,10 +28,22 @@ int pzgen_3(const PairGeom& g, const float2* tw, float2* S, const OtfDev& otf, b
       return pz_mode<PPZ147, 8>(g, tw, S, otf, conj, st, fwd_only);
     case 192:
       *done = true;
-      return pz_mode<PPZ192, 16>(g, tw, S, otf, conj, st, fwd_only);
+      return pz_mode<PPZ192, 8>(g, tw, S, otf, conj, st, fwd_only);
     case 243:
       *done = true;
       return pz_mode<PPZ243, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 294:
+      *done = true;
+      return pz_mode<PPZ294, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 360:
+      *done = true;
+      return pz_mode<PPZ360, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 432:
+      *done = true;
+      return pz_mode<PPZ432, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 504:
+      *done = true;
+      return pz_mode<PPZ504, 8>(g, tw, S, otf, conj, st, fwd_only);
     default:
       return 0;
   }

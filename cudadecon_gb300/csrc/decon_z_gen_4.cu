@@ -1,5 +1,5 @@
 // Generated by cudadecon_gb300/gen_plans.py (do not edit): paired z-pass kernels
-// of the lengths 24, 40, 60, 84, 120, 150, 196, 245.
+// of the lengths 24, 40, 60, 84, 120, 150, 196, 245, 300, 375, 441, 512.
 #include "decon_pz.cuh"
 #include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
@@ -25,13 +25,25 @@ int pzgen_4(const PairGeom& g, const float2* tw, float2* S, const OtfDev& otf, b
       return pz_mode<PPZ120, 16>(g, tw, S, otf, conj, st, fwd_only);
     case 150:
       *done = true;
-      return pz_mode<PPZ150, 16>(g, tw, S, otf, conj, st, fwd_only);
+      return pz_mode<PPZ150, 8>(g, tw, S, otf, conj, st, fwd_only);
     case 196:
       *done = true;
-      return pz_mode<PPZ196, 16>(g, tw, S, otf, conj, st, fwd_only);
+      return pz_mode<PPZ196, 8>(g, tw, S, otf, conj, st, fwd_only);
     case 245:
       *done = true;
       return pz_mode<PPZ245, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 300:
+      *done = true;
+      return pz_mode<PPZ300, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 375:
+      *done = true;
+      return pz_mode<PPZ375, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 441:
+      *done = true;
+      return pz_mode<PPZ441, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 512:
+      *done = true;
+      return pz_mode<PPZ512, 8>(g, tw, S, otf, conj, st, fwd_only);
     default:
       return 0;
   }

@@ -1,5 +1,5 @@
 // Generated by cudadecon_gb300/gen_plans.py (do not edit): paired z-pass kernels
-// of the lengths 25, 42, 63, 90, 125, 160, 200, 250.
+// of the lengths 25, 42, 63, 90, 125, 160, 200, 250, 315, 378, 448.
 #include "decon_pz.cuh"
 #include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
@@ -25,13 +25,22 @@ int pzgen_5(const PairGeom& g, const float2* tw, float2* S, const OtfDev& otf, b
       return pz_mode<PPZ125, 16>(g, tw, S, otf, conj, st, fwd_only);
     case 160:
       *done = true;
-      return pz_mode<PPZ160, 16>(g, tw, S, otf, conj, st, fwd_only);
+      return pz_mode<PPZ160, 8>(g, tw, S, otf, conj, st, fwd_only);
     case 200:
       *done = true;
-      return pz_mode<PPZ200, 16>(g, tw, S, otf, conj, st, fwd_only);
+      return pz_mode<PPZ200, 8>(g, tw, S, otf, conj, st, fwd_only);
     case 250:
       *done = true;
       return pz_mode<PPZ250, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 315:
+      *done = true;
+      return pz_mode<PPZ315, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 378:
+      *done = true;
+      return pz_mode<PPZ378, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 448:
+      *done = true;
+      return pz_mode<PPZ448, 8>(g, tw, S, otf, conj, st, fwd_only);
     default:
       return 0;
   }

@@ -1,5 +1,5 @@
 // Generated by cudadecon_gb300/gen_plans.py (do not edit): paired z-pass kernels
-// of the lengths 27, 45, 64, 96, 126, 162, 210, 252.
+// of the lengths 27, 45, 64, 96, 126, 162, 210, 252, 320, 384, 450.
 #include "decon_pz.cuh"
 #include "pair_plans_gen.cuh"
 #include "x_gen_dispatch.h"
@@ -28,10 +28,19 @@ int pzgen_6(const PairGeom& g, const float2* tw, float2* S, const OtfDev& otf, b
       return pz_mode<PPZ162, 8>(g, tw, S, otf, conj, st, fwd_only);
     case 210:
       *done = true;
-      return pz_mode<PPZ210, 16>(g, tw, S, otf, conj, st, fwd_only);
+      return pz_mode<PPZ210, 8>(g, tw, S, otf, conj, st, fwd_only);
     case 252:
       *done = true;
-      return pz_mode<PPZ252, 16>(g, tw, S, otf, conj, st, fwd_only);
+      return pz_mode<PPZ252, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 320:
+      *done = true;
+      return pz_mode<PPZ320, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 384:
+      *done = true;
+      return pz_mode<PPZ384, 8>(g, tw, S, otf, conj, st, fwd_only);
+    case 450:
+      *done = true;
+      return pz_mode<PPZ450, 8>(g, tw, S, otf, conj, st, fwd_only);
     default:
       return 0;
   }

@@ -5,7 +5,7 @@ csrc/static_plans.cuh does not already hold: x in [128, 1024], y in
 
 Writes csrc/static_plans_gen.cuh (those plan lists), and for the paired passes
 of the plain form (csrc/fft_pair.cuh; x in [128, 2048], y in [8, 2048], z in
-[16, 256]) csrc/pair_plans_gen.cuh (the plans), csrc/x_gen_dispatch.h (their
+[16, 512]) csrc/pair_plans_gen.cuh (the plans), csrc/x_gen_dispatch.h (their
 dispatch) and csrc/decon_{x,y,z}_gen_<k>.cu (their kernels, spread over several
 units so that the build compiles them in parallel).
 
@@ -320,7 +320,7 @@ def choose(axis: str, L: int, column: int | None,
 # ---------------------------------------------------------------- paired plans
 PAIR_X_RANGE = (128, 2048)
 PAIR_Y_RANGE = (8, 2048)
-PAIR_Z_RANGE = (16, 256)
+PAIR_Z_RANGE = (16, 512)
 PAIR_MAX_RADIX = 16
 PAIR_Y_RADIX = 18  # y 324 as 18 9 took 30-37 us a pass on 108 x 324 x 525, as 6 9 3 35-44 us
 PAIR_X_RADIX = 12  # x 256 as 4 8 8 took 17 us in x ratio, as 16 16 30 us
@@ -470,7 +470,8 @@ def pair_plan(axis: str, L: int) -> tuple[int, int, tuple[int, int, int], int, i
     keeps more warps on an SM (810 at 180 slices of 600 rows: x ratio 308 us
     with 4, 390 with 2; 1024: 282 and 234); y: neighbouring kx for about 128 threads
     at even heights; z: 16 column pairs
-    (256-byte runs), 8 where that keeps more warps on an SM."""
+    (256-byte runs), 8 past 144 slices (210: 47 us a pass with 8, 51 with 16 and 55 with
+    4 on 210 x 256 x 384) or where that keeps more warps on an SM, 4 where 8 do not fit."""
     if axis == "x":
         rad = pair_radices(L, False, PAIR_X_RADIX)
         V = 4 if pair_x_warps(L, rad, 4) > 1.1 * pair_x_warps(L, rad, 2) else 2
@@ -490,7 +491,14 @@ def pair_plan(axis: str, L: int) -> tuple[int, int, tuple[int, int, int], int, i
                 V = 2
         return (n, V, rad, *pair_strides(n, rad, V, "y", n == L))
     rad = pair_radices(L, False)
-    V = 8 if pair_z_warps(L, rad, 8) > 1.2 * pair_z_warps(L, rad, 16) else 16
+    # two radices to 24 (25 past 300) where three leave few columns a block: 147 as
+    # 21 7 took 41 us on 147 x 256 x 384, as 7 7 3 51 us; 384 as 24 16 82, as 8 8 6
+    # 111; but 175 as 25 7 62, as 5 7 5 50
+    if rad[1] > 1:
+        rad = pair_two(L, 25 if L > 300 else 24) or rad
+    V = 8 if L > 144 or pair_z_warps(L, rad, 8) > 1.2 * pair_z_warps(L, rad, 16) else 16
+    if not pair_z_warps(L, rad, V):
+        V = 4
     return (L, V, rad, rad[1] * rad[2], L)
 
 

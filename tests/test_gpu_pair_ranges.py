@@ -4,7 +4,7 @@
   other plain transforms are held to): heights of 8 to 31 and above 1024, odd
   ones of two wide and of three radices, with and without room for whole slot
   blocks (189, 225), beside even and odd depths; heights left to the generic
-  engine.
+  engine; depths above 256 and of two wide radices.
 * The convolution, which takes the columns in the order the forward y pass
   leaves them, with a radial and with a full 3D OTF: same bound.
 """
@@ -22,7 +22,8 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(6, 8, 128), (5, 9, 135), (4, 12, 128), (7, 14, 128), (3, 10, 140), (6, 15, 128), (5, 27, 150),
           (4, 28, 128), (3, 30, 128), (3, 189, 128), (2, 225, 128), (5, 375, 128), (3, 525, 135),
           (2, 875, 128), (3, 1029, 128), (2, 1080, 128), (3, 1225, 128), (2, 1458, 128), (1, 1875, 128),
-          (2, 2025, 128), (3, 2048, 128), (2, 2160, 128)]
+          (2, 2025, 128), (3, 2048, 128), (2, 2160, 128), (147, 12, 128), (175, 9, 128), (343, 8, 128),
+          (500, 9, 128), (512, 8, 128), (525, 8, 128)]
 
 
 def _dev(torch, x):
@@ -58,7 +59,7 @@ def test_transform_and_convolution(cdx, oracle, torch_cuda, tmp_path, shape):
 
 
 @pytest.mark.parametrize("shape", [(8, 27, 128), (6, 36, 135), (5, 10, 128), (3, 189, 128), (4, 225, 128),
-                                   (8, 50, 128)])
+                                   (300, 9, 128), (8, 50, 128)])
 @pytest.mark.parametrize("conj", [0, 1])
 def test_convolution_with_a_3d_otf(cdx, oracle, torch_cuda, tmp_path, shape, conj):
     torch = torch_cuda
