@@ -438,7 +438,8 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
   copy_twiddles<P::kTw>(tw, stw);
   cp_async_commit();
   const RowRuns<NQ> runs(g, z, m0);
-  const bool vec = Y && runs.vec(Xout) && runs.vec(Y) && runs.vec(G);
+  // (the halves of the rows in shared memory are 2 NQ L floats apart)
+  const bool vec = NQ * PL::L % 2 == 0 && Y && runs.vec(Xout) && runs.vec(Y) && runs.vec(G);
   // Y and G were written by kernels that completed before the previous pass
   // passed its own wait: ask for them now, in shared memory (the first STAGED of
   // them) or in L2 (16-byte walk only: the prefetch takes whole 16-byte units)

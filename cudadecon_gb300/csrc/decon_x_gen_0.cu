@@ -22,7 +22,7 @@ int pxgen_fwd_0(const PairGeom& g, const float2* tw, const float* X, float* Xm1,
       return px_fwd_go<PPX600, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 875:
       *done = true;
-      return px_fwd_go<PPX875, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
+      return px_fwd_go<PPX875, 3>(g, tw, X, Xm1, lam, predict, bg, S, st);
     case 1215:
       *done = true;
       return px_fwd_go<PPX1215, 2>(g, tw, X, Xm1, lam, predict, bg, S, st);
@@ -50,7 +50,7 @@ int pxgen_ratio_0(const PairGeom& g, const float2* tw, float2* S, const float* r
       return px_ratio_go<PPX600, 2>(g, tw, S, raw, mean, eps, st);
     case 875:
       *done = true;
-      return px_ratio_go<PPX875, 2>(g, tw, S, raw, mean, eps, st);
+      return px_ratio_go<PPX875, 3>(g, tw, S, raw, mean, eps, st);
     case 1215:
       *done = true;
       return px_ratio_go<PPX1215, 2>(g, tw, S, raw, mean, eps, st);
@@ -78,7 +78,7 @@ int pxgen_update_0(const PairGeom& g, const float2* tw, const float2* S, const f
       return px_update_go<PPX600, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
     case 875:
       *done = true;
-      return px_update_go<PPX875, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
+      return px_update_go<PPX875, 3>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);
     case 1215:
       *done = true;
       return px_update_go<PPX1215, 2>(g, tw, S, Y, Xout, G, dots, w, lam_next, eps, st);

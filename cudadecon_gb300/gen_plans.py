@@ -474,6 +474,11 @@ def pair_plan(axis: str, L: int) -> tuple[int, int, tuple[int, int, int], int, i
     4 on 210 x 256 x 384) or where that keeps more warps on an SM, 4 where 8 do not fit."""
     if axis == "x":
         rad = pair_radices(L, False, PAIR_X_RADIX)
+        if max(rad) > 16 and rad[1] > 1 and (pair_two(L, PAIR_WIDE_RADIX) or (0, 0, 99))[2] <= 25:
+            # 875 as 35 25 with 3 pairs: 548 us an iteration of 100 x 225 x 875; as 7 25 5
+            # 600 to 650 us (one block an SM), as 35 25 with 2 or 4 pairs 580 and 570 us
+            rad = pair_two(L, PAIR_WIDE_RADIX)
+            return (L, 3, rad, *pair_strides(L, rad, 3, "x", False))
         V = 4 if pair_x_warps(L, rad, 4) > 1.1 * pair_x_warps(L, rad, 2) else 2
         return (L, V, rad, *pair_strides(L, rad, V, "x", False))
     if axis == "y":

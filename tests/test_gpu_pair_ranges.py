@@ -7,6 +7,8 @@
   engine; depths above 256 and of two wide radices.
 * The convolution, which takes the columns in the order the forward y pass
   leaves them, with a radial and with a full 3D OTF: same bound.
+* RL at 875 columns (three pairs a block) on rows whose last block starts and
+  ends on 16 bytes: relative L2 <= 5e-6, the bound of the other paired loops.
 """
 
 import ctypes
@@ -85,3 +87,23 @@ def test_convolution_with_a_3d_otf(cdx, oracle, torch_cuda, tmp_path, shape, con
     H = np.asarray(oracle.otf_on_grid(st, nx, ny, nz, dtype=np.float32)).reshape(S.shape)
     want = np.fft.irfftn(S * (np.conj(H) if conj else H), s=shape, axes=(0, 1, 2))
     assert rel_l2(out.cpu().numpy(), want) < 2e-6
+
+
+@pytest.mark.parametrize("shape", [(8, 32, 875), (6, 27, 875), (5, 30, 875)])
+def test_rl_with_three_pairs_a_block(cdx, oracle, torch_cuda, tmp_path, shape):
+    raw = synth.bead_stack(shape, n_beads=60, psf_sigma_xy=1.3, psf_sigma_z=2.0, seed=sum(shape))
+    tab = synth.gaussian_otf_table(65, 32, 1.3, 2.5)
+    p = tmp_path / "otf.tif"
+    synth.write_otf(p, tab)
+    kw = dict(dr=0.104, dz=0.3, dr_psf=0.104, dz_psf=0.25)
+    cdx.rl_init(raw.shape, p, **kw)
+    assert cdx.decon_grid() == shape
+    mine = cdx.rl_decon(raw, background=100.0, n_iters=5)
+    cdx.rl_cleanup()
+    nz, ny, nx = shape
+    st = oracle.rl_init(nx, ny, nz, kw["dr"], kw["dz"], kw["dr_psf"], kw["dz_psf"], 0.0, 0.0, 0,
+                        False, synth.otf_table_to_image(tab))
+    X0 = oracle.bgsub(raw.astype(np.float32), 100.0)
+    want = oracle.rl_iterations(X0, X0, oracle.otf_on_grid(st, nx, ny, nz, dtype=np.float64), 5,
+                                dtype=np.float64)
+    assert rel_l2(mine, want) < 5e-6
