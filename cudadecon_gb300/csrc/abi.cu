@@ -64,6 +64,9 @@ static unsigned find_optimal_dimension(unsigned in, int step = -1) {
 }
 
 // ---------------------------------------------------------------- device buffers
+// Give back what the session keeps only to save time (false: nothing kept).
+static bool release_kept();
+
 template <class T>
 struct DevBuf {
   T* p = nullptr;
@@ -75,6 +78,10 @@ struct DevBuf {
     n = 0;
     if (count == 0) return 0;
     cudaError_t e = cudaMalloc(&p, sizeof(T) * count);
+    if (e == cudaErrorMemoryAllocation && release_kept()) {
+      cudaGetLastError();
+      e = cudaMalloc(&p, sizeof(T) * count);
+    }
     if (e != cudaSuccess) {
       p = nullptr;
       set_cuda_error("cudaMalloc", e);
@@ -137,6 +144,7 @@ struct Session {
   // Wiener filter: spectrum, filter factors, background-subtracted volume
   DevBuf<float2> wiener_S, wiener_H;
   DevBuf<float> wiener_in;
+  bool wiener_busy = false;  // a call is using them
   void release_wiener() {
     wiener_S.release();
     wiener_H.release();
@@ -163,6 +171,14 @@ struct Session {
 };
 
 static Session g_s;
+
+// The Wiener filter's workspaces: an allocation that fails gets their memory.
+static bool release_kept() {
+  Session& s = g_s;
+  if (s.wiener_busy || !(s.wiener_S.p || s.wiener_H.p || s.wiener_in.p)) return false;
+  s.release_wiener();
+  return true;
+}
 static std::mutex g_mu;
 
 // Optional per-pass timing with CUDA events recorded on the launch stream
@@ -1773,7 +1789,7 @@ int cdx_wiener_device(const float* in, float* out, int nx, int ny, int nz, float
   const float w = wiener * wiener;
   const float kxscale = dkx / s.dkx_otf, kyscale = dky / s.dkx_otf, kzscale = dkz / s.dkz_otf;
   // The workspaces stay with the session up to kWienerKeep bytes, until
-  // RL_cleanup: at 100x256x756 the passes take 280 us, and allocating and
+  // RL_cleanup or until an allocation fails (release_kept): at 100x256x756 the passes take 280 us, and allocating and
   // freeing the three around them took another 440 us.  Every call ends
   // synchronised, so calls on different streams can share them.
   constexpr size_t kWienerKeep = 4ull << 30;
@@ -1781,6 +1797,7 @@ int cdx_wiener_device(const float* in, float* out, int nx, int ny, int nz, float
   OtfDev hd{};
   // the paired x pass subtracts the background as it reads (one pass over the
   // volume less: 280 us become 247)
+  s.wiener_busy = true;
   int ok = !(s.wiener_S.ensure(ns) || s.wiener_H.ensure(ns) ||
              (!g.pair && s.wiener_in.ensure(nv)));
   if (ok) {
@@ -1797,6 +1814,7 @@ int cdx_wiener_device(const float* in, float* out, int nx, int ny, int nz, float
     // also after a failure: earlier passes may still be using the workspaces
     ok = cudaStreamSynchronize(st) == cudaSuccess && ok;
   }
+  s.wiener_busy = false;
   const size_t held =
       sizeof(float2) * (s.wiener_S.n + s.wiener_H.n) + sizeof(float) * s.wiener_in.n;
   if (!ok || held > kWienerKeep) s.release_wiener();
