@@ -1,15 +1,17 @@
 """Autotuner of the generated compile-time FFT plans.
 
-Every length of the batched workloads' ranges has a few candidate plans
-(gen_plans.candidates): radix order, pencil batch (y rows, z columns or x
-row pairs per block), register budget and stage-layout padding.  Plans are compile-time types,
-so the tuner builds the library once per candidate column (column k =
-candidate k of every length, candidate 0 where a length has fewer) in a
-scratch copy of the package, runs one synthetic stack per length through cdx_RL_device with the
-per-pass timers (cdx_profile_*) on this GPU, and keeps, per axis and length,
-the candidate with the shortest pass time: x = forward + ratio + update
-passes, y = the four y passes, z = the two z passes of an iteration.  A
-candidate replaces candidate 0 only when it is faster by more than the
+Every y and z length of the batched workloads' ranges has a few candidate plans
+(gen_plans.candidates): radix order, pencil batch (y rows or z columns per
+block), register budget and stage-layout padding.  They are the plans of the
+plain spectrum layout, which the mixed-precision form uses at the widths of its
+tensor-core x passes; the paired passes of the plain form have plans of their
+own (gen_plans.pair_plan), which are not tuned here.  Plans are compile-time
+types, so the tuner builds the library once per candidate column (column k =
+candidate k of every length, candidate 0 where a length has fewer) in a scratch
+copy of the package, runs one synthetic stack per length through cdx_RL_device
+in the mixed form with the per-pass timers (cdx_profile_*) on this GPU, and
+keeps, per axis and length, the candidate with the shortest pass time: y = the
+four y passes, z = the two z passes of an iteration.  A candidate replaces candidate 0 only when it is faster by more than the
 margin (timing noise).  The choices and the measured times are written to
 tuned_plans.json, then gen_plans.py regenerates the plan sources from it;
 rebuild the library afterwards.
@@ -18,8 +20,8 @@ rebuild the library afterwards.
                                        [--workdir DIR] [--no-apply]
 
 The stack of probe i has z, y and x lengths zs[i % nz], ys[i % ny] and
-xs[i % nx], so every length is timed at least once on its axis; every
-column times the same stacks.
+xs[i % nx], so every length is timed at least once on its axis (x: the
+tensor-core widths); every column times the same stacks.
 """
 
 from __future__ import annotations
@@ -40,6 +42,14 @@ ROOT = PKG.parent
 # y_inv, x_ratio_fwd, y_fwd2, z_otf_conj, y_inv2, x_inv_update)
 AXIS_PASSES = {"x": (0, 4, 8), "y": (1, 3, 5, 7), "z": (2, 6)}
 ITERS = 10
+# widths of the tensor-core x passes (CDX_TC_PLANS, csrc/decon_x_tc.cu): the mixed
+# form runs the tuned y and z plans there
+TC_WIDTHS = [256, 512, 756, 1024]
+
+
+def tuned_lengths(lens: dict[str, list[int]]) -> dict[str, list[int]]:
+    """The lengths whose plans are tuned, and the widths they are tuned at."""
+    return {"x": TC_WIDTHS, "y": lens["y"], "z": lens["z"]}
 
 
 def probe_shapes(lens: dict[str, list[int]]) -> list[tuple[int, int, int]]:
@@ -99,6 +109,7 @@ def run_probe(shapes, out_path: Path) -> None:
     torch.cuda.set_device(0)
     dev = torch.device("cuda", 0)
     L = cdx.lib()
+    cdx.set_dft_form("mixed")
     stream = torch.cuda.Stream(device=dev)
     sp = ctypes.c_void_p(stream.cuda_stream)
     td = tempfile.TemporaryDirectory()
@@ -156,7 +167,7 @@ def tune(columns: int, margin: float, workdir: Path, apply: bool) -> dict:
     sys.path.insert(0, str(PKG))
     import gen_plans as G
 
-    lens = G.lengths()
+    lens = tuned_lengths(G.lengths())
     shapes = probe_shapes(lens)
     times = []
     device = None
@@ -184,7 +195,7 @@ def tune(columns: int, margin: float, workdir: Path, apply: bool) -> dict:
         device = d["device"]
         t = axis_times([tuple(r["shape"]) for r in d["rows"]], [r["pass_ms"] for r in d["rows"]],
                        lens)
-        times.append(t)
+        times.append(dict(t, x={}))
         tot = sum(sum(v.values()) for v in t.values())
         print(f"column {k}: {len(d['rows'])} stacks, {tot:.3f} ms of pass time per iteration",
               flush=True)

@@ -23,8 +23,8 @@ between the stages); candidate 0 is the heuristic choice:
          radices (the most balanced triple) with the full and half batch:
          an unbalanced pair such as 125 = 25*5 leaves most threads idle in
          its large-radix stage.
-  x    : (chosen and tuned, but compiled into nothing: the paired passes took
-         over every x length of a plan)
+  x    : (neither tuned nor compiled: the paired passes took over every x
+         length of a plan)
          the most balanced three radices, smallest last (the fused epilogues
          of the x passes run in the last stage, which then has a thread for
          every butterfly), with the generic engine's row pairs per block.
@@ -39,8 +39,9 @@ by a model of the shared-memory bank conflicts of the stage that writes it
 and the stage that reads it (smem_pads); one candidate per length carries
 the model's padding where the model finds one.
 
-autotune.py times the candidates on the GPU and records the fastest per
-axis and length in tuned_plans.json, which this script then follows.
+autotune.py times the y and z candidates on the GPU, in the mixed-precision
+form that runs them, and records the fastest per axis and length in
+tuned_plans.json, which this script then follows.
 
     python cudadecon_gb300/gen_plans.py               (tuned, else candidate 0)
     python cudadecon_gb300/gen_plans.py --column k    (candidate k everywhere,
