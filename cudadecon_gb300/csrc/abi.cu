@@ -391,8 +391,8 @@ static int ensure_plan(Session& s, int gx, int gy, int gz) {
 
 // Floats of LoopBufs::lam: two lambda slots, the means taken off the first, the
 // second and the later ratios, and those means convolved.  All 0 at the start of a
-// loop.
-constexpr int kLoopScalars = 8;
+// loop.  The means have a cache line of their own: lambda is written every iteration.
+constexpr int kLoopMeans = 32, kLoopScalars = kLoopMeans + 6;
 
 static int ensure_grid_buffers(Session& s, const Geom& g) {
   const size_t n = (size_t)g.nvox();
@@ -459,8 +459,8 @@ static int rl_loop(const GridPlan& p, const LoopBufs& b, int nIter, cudaStream_t
     mark();
     // nothing is taken off the first ratio, the first ratio's mean off the second,
     // the second's off all that follow (measured anew each time the error is the same)
-    conj.mean = b.lam + 2 + std::min(k, 2);
-    conj.mean_next = k < 2 ? b.lam + 3 + k : nullptr;
+    conj.mean = b.lam + kLoopMeans + std::min(k, 2);
+    conj.mean_next = k < 2 ? b.lam + kLoopMeans + 1 + k : nullptr;
     w.add = conj.mean + 3;
     if ((rc = launch_x_inv_ratio_fwd(g, p.fx, b.S, b.raw, conj.mean, eps, st))) return rc;
     mark();

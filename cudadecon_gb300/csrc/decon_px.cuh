@@ -29,7 +29,7 @@ struct RowQuad {
 };
 __device__ __forceinline__ RowQuad row_quad(const PairGeom& g, int z, int m) {
   RowQuad r;
-  r.o = ((long long)z * g.ny + 2 * m) * g.nx;
+  r.o = ((long long)z * g.zrows + 2 * m) * g.nx;
   r.h = (long long)g.H * g.nx;
   r.v2 = 2 * m + g.H < g.ny;
   r.v3 = 2 * m + 1 + g.H < g.ny;
@@ -41,7 +41,7 @@ __device__ __forceinline__ RowQuad row_quad(const PairGeom& g, int z, int m) {
 template <int NQ>
 __device__ __forceinline__ void prefetch_rows(const PairGeom& g, float* dst, const float* src,
                                               int z, int m0) {
-  const long long o = ((long long)z * g.ny + 2 * m0) * g.nx;
+  const long long o = ((long long)z * g.zrows + 2 * m0) * g.nx;
   const int n0 = max(0, min(2 * NQ, g.H - 2 * m0)), n1 = max(0, min(n0, g.ny - g.H - 2 * m0));
   prefetch_floats(dst, src + o, n0 * g.nx, true);
   prefetch_floats(dst + 2 * NQ * g.nx, src + o + (long long)g.H * g.nx, n1 * g.nx, true);
@@ -58,7 +58,7 @@ struct RowRuns {
   long long o, h;  // first run, distance to the second
   int n0, n1;      // floats
   __device__ __forceinline__ RowRuns(const PairGeom& g, int z, int m0) {
-    o = ((long long)z * g.ny + 2 * m0) * g.nx;
+    o = ((long long)z * g.zrows + 2 * m0) * g.nx;
     h = (long long)g.H * g.nx;
     const int r0 = max(0, min(2 * NQ, g.H - 2 * m0));
     n0 = r0 * g.nx;
@@ -349,7 +349,7 @@ k_px_ratio(PairGeom g, const float2* __restrict__ tw, float4* S, const float* __
   extern __shared__ __align__(16) float2 smem[];
   float2* stw = smem;
   float4* sm = P::tile(smem);
-  const int z = slice_of_block(g), m0 = blockIdx.x * NQ;
+  const int z = blockIdx.y, m0 = blockIdx.x * NQ;
   copy_twiddles<P::kTw>(tw, stw);
   prefetch_rows<NQ>(g, P::rows(smem, 0), raw, z, m0);  // written before the iterations
   cp_async_commit();
@@ -434,7 +434,7 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
   __shared__ float4 red[32];
   float2* stw = smem;
   float4* sm = P::tile(smem);
-  const int z = slice_of_block(g), m0 = blockIdx.x * NQ;
+  const int z = blockIdx.y, m0 = blockIdx.x * NQ;
   copy_twiddles<P::kTw>(tw, stw);
   cp_async_commit();
   const RowRuns<NQ> runs(g, z, m0);
@@ -509,23 +509,26 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
   }
   if (vec) {
     constexpr int U = 2;  // accesses in flight per thread and array
-    const int n0 = runs.n0 >> 2, n = total >> 2;
-    const long long o0 = runs.o >> 2, o1 = ((runs.o + runs.h) >> 2) - n0;
+    // from the block's first row, which is what lies on 16 bytes
+    const int n0 = runs.n0 >> 2, n = total >> 2, o1 = (int)(runs.h >> 2) - n0;
+    const float4* Y4 = reinterpret_cast<const float4*>(Y + runs.o);
+    float4* X4 = reinterpret_cast<float4*>(Xout + runs.o);
+    float4* G4 = reinterpret_cast<float4*>(G + runs.o);
     const float4* r4 = reinterpret_cast<const float4*>(rows);
     for (int i0 = idx; i0 < n; i0 += U * P::T) {
       float4 y[U], go[U];
-      long long at[U];
+      int at[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int i = i0 + u * P::T;
-        at[u] = (i < n0 ? o0 : o1) + i;
+        at[u] = i < n0 ? i : o1 + i;
         if (i < n) {
           const int f = i < n0 ? i : i - n0 + NQ * PL::L / 2;
           y[u] = STAGED > 0 ? reinterpret_cast<const float4*>(P::rows(smem, 0))[f]
-                            : __ldcs(reinterpret_cast<const float4*>(Y) + at[u]);
+                            : __ldcs(Y4 + at[u]);
           if (dots)
             go[u] = STAGED > 1 ? reinterpret_cast<const float4*>(P::rows(smem, 1))[f]
-                               : __ldcs(reinterpret_cast<const float4*>(G) + at[u]);
+                               : __ldcs(G4 + at[u]);
         }
       }
 #pragma unroll
@@ -538,8 +541,8 @@ k_px_update(PairGeom g, const float2* __restrict__ tw, float4* S, const float* Y
                ga);
         update(make_float2(c.z, c.w), make_float2(y[u].z, y[u].w), make_float2(go[u].z, go[u].w), xb,
                gb);
-        reinterpret_cast<float4*>(Xout)[at[u]] = make_float4(xa.x, xa.y, xb.x, xb.y);
-        __stcs(reinterpret_cast<float4*>(G) + at[u], make_float4(ga.x, ga.y, gb.x, gb.y));
+        X4[at[u]] = make_float4(xa.x, xa.y, xb.x, xb.y);
+        __stcs(G4 + at[u], make_float4(ga.x, ga.y, gb.x, gb.y));
       }
     }
   } else {

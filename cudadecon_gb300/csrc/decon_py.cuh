@@ -83,7 +83,7 @@ k_py_eo(PairGeom g, const float2* __restrict__ tw, float4* S) {
   copy_twiddles<P::kTw>(tw, stw);
   cp_async_commit();
   const int idx = threadIdx.x, kx0 = blockIdx.x * V;
-  float4* slice = S + (long long)slice_of_block(g) * g.zstep;
+  float4* slice = S + (long long)blockIdx.y * g.zstep;
   // slot s + r STEP of row kx; whole blocks of 4 slots apart for the usual STEP
   auto slot = [&](int kx, int s, auto stepc, int r) {
     constexpr int STEP = decltype(stepc)::value;
@@ -287,7 +287,7 @@ k_py_zz(PairGeom g, const float2* __restrict__ tw, float4* S) {
   cp_async_commit();
   grid_dep_wait();
   // slices z0 and z0 + 1 (the last of an odd count stands alone)
-  const int z0 = 2 * slice_of_block(g), kx0 = blockIdx.x * V, idx = threadIdx.x;
+  const int z0 = 2 * blockIdx.y, kx0 = blockIdx.x * V, idx = threadIdx.x;
   const bool two = z0 + 1 < g.nz;
   float4* slice = S + (long long)z0 * g.zstep;
   const long long dz = two ? g.zstep : 0;

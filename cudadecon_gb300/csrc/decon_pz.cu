@@ -61,7 +61,7 @@ k_pz_gen(PairGeom g, FftDev fz, float4* S, OtfDev otf, int conj, int fwd_only, i
   float* car = reinterpret_cast<float*>(cir + W);
   load_twiddles(fz, stw);
   for (int v = threadIdx.x; v < W; v += blockDim.x) {
-    const int f = f0 + (v >> 1), kx = f >> 2, s = blockIdx.y * 4 + (f & 3), y = g.col(s, v & 1);
+    const int f = f0 + (v >> 1), kx = f >> 2, s = blockIdx.y * 4 + (f & 3), y = g.col(s) + (v & 1) * g.col_step(s);
     int ir = -1;
     float ar = 0.f;
     if (kx < g.nxh && s < g.slots && y < g.ny && otf.mode == 0) {

@@ -141,7 +141,7 @@ k_pz(PairGeom g, const float2* __restrict__ tw, float4* S, OtfDev otf, int conj,
           // per kz (dev_otfinterpolate RA branch, RLgpuImpl.cu:238-273)
           int ir0 = 0, ir1 = 0;
           float ar0 = 0.f, ar1 = 0.f;
-          const int y0 = g.col(s, 0), y1 = y0 + g.col_step(s);
+          const int y0 = g.col(s), y1 = y0 + g.col_step(s);
           const bool in0 = in && y0 < g.ny && otf_radius(otf, kx, y0, g.ny, ir0, ar0);
           const bool in1 = in && y1 < g.ny && otf_radius(otf, kx, y1, g.ny, ir1, ar1);
           const float4* t0 = otf.tz + (long long)b * otf.nr + ir0;

@@ -9,9 +9,10 @@ int launch_x_inv_ratio_fwd(const Geom& g, const FftLen& fx, float2* S, const flo
                            const float* mean, float eps, cudaStream_t st) {
   if (g.pair) {
     bool done = false;
-    PairGeom pg = pair_geom(g);
-    pg.down = past_l2(g);
-    const int rc = pxgen_ratio(pg, fx.d_pair, S, raw, mean, eps, st, &done);
+    const PairGeom up = pair_geom(g);
+    const int rc = past_l2(g) ? pxgen_ratio(pair_geom_down(g), fx.d_pair, last_slice(up, S),
+                                            last_slice_real(up, raw), mean, eps, st, &done)
+                              : pxgen_ratio(up, fx.d_pair, S, raw, mean, eps, st, &done);
     if (done || rc) return rc;
   }
   if (fx.has_tc && dft_form() == 1)

@@ -51,10 +51,13 @@ int launch_x_inv_update(const Geom& g, const FftLen& fx, const float2* S, const 
                         cudaStream_t st) {
   if (g.pair) {
     bool done = false;
-    PairGeom pg = pair_geom(g);
-    pg.down = past_l2(g);
-    const int rc = pxgen_update(pg, fx.d_pair, S, Y, Xout, G, dots, &w, lam_next, eps, st,
-                                &done);
+    const PairGeom up = pair_geom(g);
+    const int rc =
+        past_l2(g)
+            ? pxgen_update(pair_geom_down(g), fx.d_pair, last_slice(up, const_cast<float2*>(S)),
+                           last_slice_real(up, Y), last_slice_real(up, Xout),
+                           last_slice_real(up, G), dots, &w, lam_next, eps, st, &done)
+            : pxgen_update(up, fx.d_pair, S, Y, Xout, G, dots, &w, lam_next, eps, st, &done);
     if (done || rc) return rc;
   }
   if (fx.has_tc && dft_form() == 1)

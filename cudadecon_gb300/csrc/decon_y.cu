@@ -55,9 +55,11 @@ static int y_dispatch(const Geom& g, const FftLen& fy, float2* S, cudaStream_t s
 int launch_y_pass(const Geom& g, const FftLen& fy, float2* S, bool inverse, cudaStream_t st,
                   bool after_fwd) {
   if (g.pair) {
-    PairGeom pg = pair_geom(g);
-    pg.down = after_fwd && past_l2(g);
-    return launch_py(pg, fy, S, inverse, st);
+    const PairGeom up = pair_geom(g);
+    // (the generic form, of heights without a plan, has no order of its own)
+    if (after_fwd && past_l2(g) && fy.d_pair)
+      return launch_py(pair_geom_down(g), fy, last_slice(up, S), inverse, st);
+    return launch_py(up, fy, S, inverse, st);
   }
   return inverse ? y_dispatch<true>(g, fy, S, st) : y_dispatch<false>(g, fy, S, st);
 }

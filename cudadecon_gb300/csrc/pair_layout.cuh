@@ -40,18 +40,17 @@ struct PairGeom {
   int eo;      // 1: columns (k, k + ny/2)
   int kc;      // > 0: columns (k + 2q kc, k + (2q + 1) kc); neither: (2p, 2p + 1)
   int kcs, full;  // slots from one q to the next, slots of such pairs
-  int last;       // first of the last kc columns, less 2 full
+  int per, last, step;  // other slots: columns per s + last and step further
   float inv_kcs;
   int zstep;   // slots per z: sb * nxh * 4
-  int down = 0;  // 1: the pass takes the slices from the last to the first
-  // columns of slot s; ny and more: none.  (The quotient is exact: s + 1/2 lies
+  int zrows;   // rows of the real arrays per z: ny
+  // first column of slot s and how much further the second is; ny and more: none.  (The quotient is exact: s + 1/2 lies
   // farther from the multiples of kcs than s < 2^20 rounds.)
-  __host__ __device__ int col_step(int s) const { return eo ? ny >> 1 : s >= full ? 1 : kc; }
-  __host__ __device__ int col(int s, int lane) const {
-    if (eo) return s + lane * (ny >> 1);
-    if (s >= full) return 2 * s + lane + last;
+  __host__ __device__ int col_step(int s) const { return s < full ? kc : step; }
+  __host__ __device__ int col(int s) const {
+    if (s >= full) return per * s + last;
     const int q = (int)(((float)s + 0.5f) * inv_kcs), k = s - q * kcs;
-    return k < kc ? k + (2 * q + lane) * kc : ny;
+    return k < kc ? k + 2 * q * kc : ny;
   }
   // slot s of row (kx, z)
   __host__ __device__ long long slot(int kx, int z, int s) const {
@@ -107,18 +106,33 @@ inline PairGeom pair_geom(const Geom& g) {
   p.kc = g.kc;
   p.kcs = pair_kcs(g.ny, g.kc);
   p.full = g.kc ? (g.ny / g.kc - 1) / 2 * p.kcs : 0;
+  p.per = g.eo ? 1 : 2;
   p.last = g.kc ? g.ny - g.kc - 2 * p.full : 0;
+  p.step = g.eo ? g.ny / 2 : 1;
   p.inv_kcs = g.kc ? 1.f / (float)p.kcs : 0.f;
   if (g.kc) p.slots = p.full + (g.kc + 1) / 2;
   p.zstep = p.sb * g.nxh * 4;
+  p.zrows = g.ny;
   return p;
+}
+// The same for a pass that takes the slices from the last to the first: its kernels
+// count up from the last slice with the steps turned round, at no cost to them (a
+// choice made in the kernel took 1 of 118 us from 100x128x512).  Its arrays start at
+// the last slice.
+inline PairGeom pair_geom_down(const Geom& g) {
+  PairGeom p = pair_geom(g);
+  p.zstep = -p.zstep;
+  p.zrows = -p.zrows;
+  return p;
+}
+// Last slice of a spectrum, of a real array.
+inline float2* last_slice(const PairGeom& up, float2* S) { return S + 2LL * (up.nz - 1) * up.zstep; }
+template <class T>
+T* last_slice_real(const PairGeom& up, T* x) {
+  return x ? x + (long long)(up.nz - 1) * up.ny * up.nx : x;
 }
 
 #ifdef __CUDACC__
-// The slice (pair) of a block of a pass whose grid's y runs over them.
-__device__ __forceinline__ int slice_of_block(const PairGeom& g) {
-  return g.down ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
-}
 // Element (kx, z, ky) of a half spectrum in the layout of g.
 __device__ __forceinline__ void st_spec(const Geom& g, const PairGeom& pg, float2* S, int kx, int z,
                                         int ky, float2 v) {

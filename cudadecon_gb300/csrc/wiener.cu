@@ -70,7 +70,7 @@ __global__ void k_wiener_h_pair(Geom g, PairGeom pg, const float2* __restrict__ 
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   const int z = blockIdx.y, j = f >> 2, s = blockIdx.z * 4 + (f & 3);
   if (j >= g.nxh || s >= pg.slots) return;
-  const int y0 = pg.col(s, 0), y1 = y0 + pg.col_step(s);
+  const int y0 = pg.col(s), y1 = y0 + pg.col_step(s);
   float2 a = make_float2(0.f, 0.f), b = a;
   if (y0 < g.ny)
     a = wiener_factor(g, j, y0, z, otf, nr, nzotf, dkx, dky, kxscale, kyscale, kzscale, rcutoff, w,
