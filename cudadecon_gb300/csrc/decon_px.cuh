@@ -266,7 +266,9 @@ k_px_fwd(PairGeom g, const float2* __restrict__ tw, const float* X, float* Xm1, 
   const int idx = threadIdx.x;
   const int q = idx / PL::KC, k = idx - q * PL::KC;
   const RowQuad rq = row_quad(g, z, m0 + q);
-  const float2 lam = dup2(predict ? __ldcg(lamp) : 0.f);
+  // (a plain load: the read-only path promises that nobody writes while the kernel
+  // is resident; past L1 it takes every warp to one L2 line)
+  const float2 lam = dup2(predict ? *lamp : 0.f);
   cp_async_wait_all();
   __syncthreads();
   C2 x[PL::Q2];

@@ -13,7 +13,7 @@ namespace cdx {
 // ---------------------------------------------------------------- x forward
 template <class Run>
 __global__ void __launch_bounds__(Run::kThreads, Run::template min_blocks<6>())
-k_x_fwd(Geom g, FftDev fx, const float* __restrict__ X, float* Xm1, const float* __restrict__ lamp,
+k_x_fwd(Geom g, FftDev fx, const float* __restrict__ X, float* Xm1, const float* lamp,
         int predict, float2* __restrict__ S, int Pa) {
   const int P = tile_vectors<Run>(Pa);
   extern __shared__ __align__(16) float2 smem[];
@@ -35,7 +35,7 @@ k_x_fwd(Geom g, FftDev fx, const float* __restrict__ X, float* Xm1, const float*
   prefetch_floats(Xs, X + roff, nr * nx, true);
   if (predict) prefetch_floats(Xm1s, Xm1 + roff, nr * nx, true);
   cp_async_commit();
-  const float lam = predict ? __ldcg(lamp) : 0.f;
+  const float lam = predict ? *lamp : 0.f;  // not read-only: k_lambda may still run at the start
   cp_async_wait_all();
   __syncthreads();
   // prediction of updatePrediction_kernel (RLgpuImpl.cu:658-666), applied
