@@ -93,7 +93,8 @@ k_pz_gen(PairGeom g, FftDev fz, float4* S, OtfDev otf, int conj, int fwd_only, i
 __global__ void __launch_bounds__(32) k_ratio_mean(PairGeom g, const float4* S, OtfDev otf) {
   grid_dep_wait();
   grid_dep_launch();
-  store_ratio_mean(g, S, otf);
+  store_ratio_mean(otf, reinterpret_cast<const float*>(S), g.nz, 4LL * g.zstep, __ldcg(otf.mean),
+                   __ldg(otf.h0));
 }
 
 int launch_pz(const PairGeom& g, const FftLen& fz, float2* S, const OtfDev& otf, bool conj,

@@ -27,18 +27,16 @@ struct PZ {
 
 // The mean of the ratio whose spectrum the z pass is given, for the next iteration
 // (k_px_ratio): what was taken off it plus what is left at frequency 0, the sum of
-// column (0, 0) over z (twice the transform, as the paired passes have it).  The
-// first warp of the block that has that column calls this before it is overwritten.
-// The ratio lies within 10; a mean that does not (NaN, when the image holds one)
-// gives 0.  Kernels of their own have it (MEAN), for two passes of a loop: in the
-// others, never reached, it cost 64 x 256 x 384 0.9% of an iteration.
-__device__ __forceinline__ void store_ratio_mean(const PairGeom& g, const float4* S,
-                                                 const OtfDev& otf) {
-  const float before = __ldcg(otf.mean), h0 = __ldg(otf.h0);
+// column (0, 0) over z (twice the transform, as the paired passes have it).  One
+// warp calls this before the column is overwritten: its values lie `step` floats
+// apart from p, in shared or global memory; before, h0: what was taken off and the
+// OTF at frequency 0.  The ratio lies within 10; a mean that does not (NaN, when the
+// image holds one) gives 0.
+__device__ __forceinline__ void store_ratio_mean(const OtfDev& otf, const float* p, int nz,
+                                                 long long step, float before, float h0) {
   float sum = 0.f;
 #pragma unroll 4
-  for (int z = threadIdx.x; z < g.nz; z += 32)
-    sum += *reinterpret_cast<const float*>(S + (long long)z * g.zstep);
+  for (int z = threadIdx.x; z < nz; z += 32) sum += p[z * step];
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   if (threadIdx.x) return;
   float m = __fmaf_rn(sum, otf.inv2n, before);
@@ -87,7 +85,13 @@ k_pz(PairGeom g, const float2* __restrict__ tw, float4* S, OtfDev otf, int conj,
   int t = blockIdx.x;
   grid_dep_wait();
   if (t < ntiles) copy(t, bufs);
-  if (MEAN && blockIdx.x == 0 && threadIdx.x < 32) store_ratio_mean(g, S, otf);
+  // Kernels of their own store the ratio's mean (MEAN), for two passes of a loop: in
+  // the others, never reached, the code cost 64 x 256 x 384 0.9% of an iteration.
+  float before = 0.f, h0 = 0.f;
+  if (MEAN && blockIdx.x == 0) {
+    before = __ldcg(otf.mean);
+    h0 = __ldg(otf.h0);
+  }
   for (int half = 0; t < ntiles; t += gridDim.x, half ^= 1) {
     float4* tc = bufs + half * P::kTile + c;
     int kx, s;
@@ -96,6 +100,11 @@ k_pz(PairGeom g, const float2* __restrict__ tw, float4* S, OtfDev otf, int conj,
     float4* col = S + col_at;
     cp_async_wait_all();
     __syncthreads();
+    if (MEAN && t == 0) {  // column (0, 0) is the tile's first
+      if (threadIdx.x < 32)
+        store_ratio_mean(otf, reinterpret_cast<const float*>(bufs), PL::L, 4 * W, before, h0);
+      __syncthreads();
+    }
     if (t + gridDim.x < ntiles) copy(t + gridDim.x, bufs + (half ^ 1) * P::kTile);
     if (b < KA) {
       C2 x[Q0];
@@ -141,8 +150,13 @@ k_pz(PairGeom g, const float2* __restrict__ tw, float4* S, OtfDev otf, int conj,
           // per kz (dev_otfinterpolate RA branch, RLgpuImpl.cu:238-273)
           int ir0 = 0, ir1 = 0;
           float ar0 = 0.f, ar1 = 0.f;
-          const int y0 = g.col(s), y1 = y0 + g.col_step(s);
-          const bool in0 = in && y0 < g.ny && otf_radius(otf, kx, y0, g.ny, ir0, ar0);
+          // (a slot without columns has its first so far out that no radius reaches it)
+          int y0 = g.per * s, y1 = y0 + g.step;
+          if (g.kc) {
+            y0 = g.col(s);
+            y1 = y0 + g.col_step(s);
+          }
+          const bool in0 = in && otf_radius(otf, kx, y0, g.ny, ir0, ar0);
           const bool in1 = in && y1 < g.ny && otf_radius(otf, kx, y1, g.ny, ir1, ar1);
           const float4* t0 = otf.tz + (long long)b * otf.nr + ir0;
           const float4* t1 = otf.tz + (long long)b * otf.nr + ir1;

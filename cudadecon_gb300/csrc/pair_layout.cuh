@@ -32,6 +32,8 @@
 
 namespace cdx {
 
+constexpr int kNoColumn = 1 << 24;
+
 struct PairGeom {
   int nx, ny, nz, nxh;
   int H, hp;   // row y shares a complex row with y + H; slots per half row
@@ -44,13 +46,13 @@ struct PairGeom {
   float inv_kcs;
   int zstep;   // slots per z: sb * nxh * 4
   int zrows;   // rows of the real arrays per z: ny
-  // first column of slot s and how much further the second is; ny and more: none.  (The quotient is exact: s + 1/2 lies
+  // first column of slot s and how much further the second is; past ny: none.  (The quotient is exact: s + 1/2 lies
   // farther from the multiples of kcs than s < 2^20 rounds.)
   __host__ __device__ int col_step(int s) const { return s < full ? kc : step; }
   __host__ __device__ int col(int s) const {
     if (s >= full) return per * s + last;
     const int q = (int)(((float)s + 0.5f) * inv_kcs), k = s - q * kcs;
-    return k < kc ? k + 2 * q * kc : ny;
+    return k < kc ? k + 2 * q * kc : kNoColumn;
   }
   // slot s of row (kx, z)
   __host__ __device__ long long slot(int kx, int z, int s) const {
