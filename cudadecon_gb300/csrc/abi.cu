@@ -780,14 +780,11 @@ static int init_session(Session& s, int nx, int ny, int nz, float dr, float dz, 
 // the stacks, largest first, each go to the least-loaded of K streams forked
 // from the origin stream, so the graph holds K independent chains of about
 // equal work and small stacks run concurrently.  K is 2 by default
-// (cdx_batch_set_streams): on the 64-stack uneven batch, device-resident and
-// with the unpaired passes,
-// 1, 2, 3, 4, 6, 8 and 16 streams gave 42.7, 44.6, 43.9, 42.6, 40.2, 39.9 and
-// 39.9 G voxel-iter/s (more concurrent stacks share the L2 that holds a
-// stack's spectrum between its passes).  The host batch's transfers run on
-// an upload and a download stream of their own, so they overlap the chains
-// whatever K is: 1, 2, 3, 4 and 6 streams gave 42.7, 44.8, 44.0, 42.6 and
-// 39.2 G end to end.
+// (cdx_batch_set_streams): on the 64-stack uneven batch, device-resident, 1, 2, 3
+// and 4 streams gave 47.1, 49.0, 47.2 and 45.6 G voxel-iter/s (more concurrent
+// stacks share the L2 that holds a stack's spectrum between its passes).  The host
+// batch's transfers run on an upload and a download stream of their own, so they
+// overlap the chains whatever K is: 47.0, 49.3, 47.6 and 45.7 G end to end.
 constexpr int kBatchStreams = 16;
 static int g_batch_streams[2] = {2, 2};  // device batch, host batch
 
